@@ -463,6 +463,10 @@ QZ_API int qz_ptcl_idx_to_box_idx(int lv, int box_ts_x, int box_ts_y, int box_ts
 QZ_API int qz_test_scan(qz_sim *sim, const int *in, int *out, long n, int in_place,
                         unsigned epoch);
 QZ_API int qz_test_wait_gives_up(qz_sim *sim, int which, int *out2);
+/* qz_test_cg_ghosts: the on-chip conjugate gradient keeps at most `rows` ghost
+ * rows a block in shared memory and the others in device memory (0: as many as
+ * it makes room for); results do not depend on it. */
+QZ_API int qz_test_cg_ghosts(qz_sim *sim, int rows);
 
 #ifdef __cplusplus
 }

@@ -20,7 +20,7 @@ LIBDIR = os.path.join(HERE, "lib")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 CUDA_SOURCES = ["qz_capi.cu", "qz_particles.cu", "qz_poisson.cu", "qz_sort.cu", "qz_amr.cu",
-                "qz_noalloc.cu", "qz_observe.cu",
+                "qz_cg_resident.cu", "qz_noalloc.cu", "qz_observe.cu",
                 "qz_ensemble.cu", "qz_adjoint.cu", "qz_snapshot.cu", "qz_testhooks.cu",
                 "qz_node_mg.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -47,6 +47,7 @@ def build_cuda(force: bool = False, verbose_ptxas: bool = False) -> str:
     out = os.path.join(LIBDIR, "libqzb200.so")
     srcs = [os.path.join(CSRC, s) for s in CUDA_SOURCES]
     deps = srcs + [os.path.join(CSRC, "qz_internal.cuh"), os.path.join(CSRC, "qz_amr_dev.cuh"),
+                   os.path.join(CSRC, "qz_cg.cuh"),
                    os.path.join(ROOT, "include", "qz_b200.h")]
     if not force and not _newer(out, deps):
         return out

@@ -144,6 +144,7 @@ def load() -> C.CDLL:
         "qz_node_conjugate_gradient": ([vp] + [C.c_int] * 5 + [_I, C.c_double, C.c_int] +
                                        [_P] * 3, C.c_int),
         "qz_test_wait_gives_up": ([vp, C.c_int, _I], C.c_int),
+        "qz_test_cg_ghosts": ([vp, C.c_int], C.c_int),
     }
     for name, (args, res) in sig.items():
         f = getattr(lib, name)

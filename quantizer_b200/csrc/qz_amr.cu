@@ -41,6 +41,7 @@
 #include <string.h>
 
 #include "qz_amr_dev.cuh"
+#include "qz_cg.cuh"
 
 namespace cgrp = cooperative_groups;
 
@@ -237,12 +238,11 @@ __global__ void k_cc_roots(int ncell, const int *__restrict__ parent, int *__res
     flagged[c] = parent[c] >= 0 ? 1 : 0;
 }
 
-__global__ void k_gather_at(int m, const int *__restrict__ src, const int *__restrict__ idx,
-                            int *__restrict__ out)
+__global__ void k_gather_at(int m, const int *const *__restrict__ at, int *__restrict__ out)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m)
-        out[i] = src[idx[i]];
+    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < m)
+        out[q] = *at[q];
 }
 
 __global__ void k_zone_box_init(int nz, int *zone_box, int *zone_cells)
@@ -406,9 +406,11 @@ __device__ __forceinline__ int classify_point(const int *box, long b, long sy, l
 }
 
 // Per node, the box grid points [bmin - ts, bmax - ts + 1]^3 in box order; fl
-// holds three flag arrays (interior | boundary | simulation boundary).
+// holds three flag arrays (interior | boundary | simulation boundary); interior
+// points are marked in the bricks of the conjugate-gradient order, if given.
 __global__ void k_classify(long total, int nn, const AmrNode *__restrict__ nodes,
-                           const int *__restrict__ box, int *__restrict__ fl)
+                           const int *__restrict__ box, int *__restrict__ fl,
+                           unsigned long long *__restrict__ bricks)
 {
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total)
@@ -423,6 +425,8 @@ __global__ void k_classify(long total, int nn, const AmrNode *__restrict__ nodes
     long b = N.box_off + ii + jj * sy + kk * sz;
     int cat = classify_point(box, b, sy, sz, ii + N.ts[0], jj + N.ts[1], kk + N.ts[2], 1 << N.lv,
                              N.contact);
+    if (bricks && cat == 1)
+        brick_mark(N, ii, jj, kk, bricks);
     fl[t] = cat == 1;
     fl[total + t] = cat == 2;
     fl[2 * total + t] = cat == 3;
@@ -522,25 +526,25 @@ static bool read_ints(qz_sim *s, const int *dsrc, long count, int *out)
     return true;
 }
 
-// Reads src[idx[q]] for the host index list idx (one launch, one read-back).
-static bool read_at(qz_sim *s, const int *dsrc, const std::vector<int> &idx, int *out)
+// Reads *at[q] for every device address of the list (one launch, one read-back).
+static bool read_at(qz_sim *s, const std::vector<const int *> &at, int *out)
 {
-    const int m = (int)idx.size();
+    const int m = (int)at.size();
     if (m == 0)
         return true;
-    if (!s->gather_idx.ensure(s->mem, 2L * m) || !ensure_small(s, m))
+    if (!s->gather_idx.ensure(s->mem, 3L * m) || !ensure_small(s, 2L * m))
     {
         set_error("gather buffer");
         return false;
     }
-    memcpy(s->h_small, idx.data(), m * sizeof(int));
-    if (!check_cuda(cudaMemcpyAsync(s->gather_idx.p, s->h_small, m * sizeof(int),
+    memcpy(s->h_small, at.data(), m * sizeof(const int *));
+    if (!check_cuda(cudaMemcpyAsync(s->gather_idx.p, s->h_small, m * sizeof(const int *),
                                     cudaMemcpyHostToDevice, s->stream),
                     "gather h2d"))
         return false;
-    launch(s, QZ_PROF_TREE, 12.0 * m, k_gather_at, dim3(blocks_for(m, 256)), dim3(256), m, dsrc,
-           s->gather_idx.p, s->gather_idx.p + m);
-    return read_ints(s, s->gather_idx.p + m, m, out);
+    launch(s, QZ_PROF_TREE, 16.0 * m, k_gather_at, dim3(blocks_for(m, 256)), dim3(256), m,
+           (const int *const *)s->gather_idx.p, s->gather_idx.p + 2L * m);
+    return read_ints(s, s->gather_idx.p + 2L * m, m, out);
 }
 
 static bool upload_nodes(qz_sim *s, AmrLevel &L)
@@ -560,7 +564,7 @@ static void free_level(const MemCtx &m, AmrLevel &L)
 {
     DBuf<int> *ib[] = {&L.box, &L.cnt, &L.pos_of_box, &L.cell_seg, &L.cell_box, &L.cell_xyz,
                        &L.cell_node, &L.intr, &L.bdry, &L.simb, &L.intr_node, &L.bdry_node,
-                       &L.simb_node, &L.nint, &L.mass_range, &L.sor};
+                       &L.simb_node, &L.nint, &L.mass_range, &L.sor, &L.pos};
     for (auto *b : ib)
         b->release(m);
     DBuf<double> *db[] = {&L.gpot, &L.gpot_old, &L.gd, &L.gax, &L.gay, &L.gaz, &L.r, &L.p, &L.Ap,
@@ -568,6 +572,7 @@ static void free_level(const MemCtx &m, AmrLevel &L)
     for (auto *b : db)
         b->release(m);
     L.nodes.release(m);
+    L.row.release(m);
     L.chunks.release(m);
     L.wpot.release(m);
     L.wnodes.release(m);
@@ -591,6 +596,12 @@ void amr_free(qz_sim *s)
     s->zone_cells.release(s->mem);
     s->gather_idx.release(s->mem);
     s->seg_mass.release(s->mem);
+    s->cgr_halo.release(s->mem);
+    s->cgr_sums.release(s->mem);
+    s->brick_mask.release(s->mem);
+    s->brick_base.release(s->mem);
+    s->cgr_spill.release(s->mem);
+    s->cgr_list.release(s->mem);
     if (s->h_small)
         cudaFreeHost(s->h_small);
     s->h_small = nullptr;
@@ -759,7 +770,7 @@ int amr_build(qz_sim *s)
             return QZ_FAILURE;
         // zones = last rank + last root flag; refine cells = last slot + last flag
         int t[4];
-        if (!read_at(s, parent, {2 * nc + nc - 1, nc + nc - 1, 4 * nc + nc - 1, 3 * nc + nc - 1}, t))
+        if (!read_at(s, {zrank + nc - 1, isroot + nc - 1, slot + nc - 1, flagged + nc - 1}, t))
             return QZ_FAILURE;
         const int nz = t[0] + t[1], nzc = t[2] + t[3];
         if (nz == 0)
@@ -844,6 +855,11 @@ int amr_build(qz_sim *s)
         C.grid_total = grid_total;
         C.cell_total = cell_total;
         C.cls_total = cls_total;
+        const bool order = s->cfg.node_solver == QZ_NODE_CG && s->cfg.cg_variant == 0;
+        unsigned long long *bricks = nullptr;
+        cg_brick_layout(C);
+        if (order && cg_brick_masks(s, C, &bricks))
+            return QZ_FAILURE;
         if (!C.box.ensure(s->mem, box_total) || !C.cnt.ensure(s->mem, box_total) ||
             !C.pos_of_box.ensure(s->mem, box_total) || !C.cell_box.ensure(s->mem, cell_total) ||
             !C.cell_xyz.ensure(s->mem, 3L * cell_total) || !C.cell_node.ensure(s->mem, cell_total) ||
@@ -877,19 +893,38 @@ int amr_build(qz_sim *s)
         // grid-point lists
         int *fl = s->amr_tmp2.p, *pos = fl + 3 * cls_total;
         launch(s, QZ_PROF_TREE, 32.0 * cls_total, k_classify, dim3(blocks_for(cls_total, 256)),
-               dim3(256), cls_total, C.nnodes, C.nodes.p, C.box.p, fl);
-        if (scan_exclusive(s, fl, pos, 3 * cls_total))
+               dim3(256), cls_total, C.nnodes, C.nodes.p, C.box.p, fl, bricks);
+        if (scan_exclusive(s, fl, pos, 3 * cls_total) || (order && cg_brick_scan(s, C)))
             return QZ_FAILURE;
-        // scan values at every node's range start in each category, and the totals
-        std::vector<int> idx;
+        // scan values at every node's range start in each category, and the totals; the
+        // same of the nodes' rows in the conjugate-gradient order
+        std::vector<const int *> at;
         for (int cat = 0; cat < 3; cat++)
             for (int q = 0; q < nz; q++)
-                idx.push_back((int)(cat * cls_total + C.h[q].cls_off));
-        idx.push_back((int)(3 * cls_total - 1));
-        std::vector<int> sv(idx.size()), lastf(1);
-        if (!read_at(s, pos, idx, sv.data()) || !read_at(s, fl, {(int)(3 * cls_total - 1)}, lastf.data()))
+                at.push_back(pos + cat * cls_total + C.h[q].cls_off);
+        at.push_back(pos + 3 * cls_total - 1);
+        at.push_back(fl + 3 * cls_total - 1);
+        if (order)
+        {
+            for (int q = 0; q < nz; q++)
+                at.push_back(s->brick_base.p + C.h[q].brick_off);
+            at.push_back(s->brick_base.p + C.brick_total - 1);
+            at.push_back(s->brick_base.p + 2 * C.brick_total - 1);
+        }
+        std::vector<int> sv(at.size());
+        if (!read_at(s, at, sv.data()))
             return QZ_FAILURE;
-        const int total_all = sv.back() + lastf[0];
+        const int total_all = sv[3 * nz] + sv[3 * nz + 1];
+        if (order)
+        {
+            const int *rv = &sv[3 * nz + 2];
+            C.row_total = rv[nz] + rv[nz + 1];
+            for (int q = 0; q < nz; q++)
+            {
+                C.h[q].row_off = rv[q];
+                C.h[q].nrows = (q + 1 < nz ? rv[q + 1] : C.row_total) - rv[q];
+            }
+        }
         auto start = [&](int cat, int q) {
             if (q < nz)
                 return sv[cat * nz + q];
@@ -924,6 +959,9 @@ int amr_build(qz_sim *s)
         if (n > 0)
             launch(s, QZ_PROF_TREE, 36.0 * n, k_next_node, dim3(blocks_for(n, 256)), dim3(256), n,
                    s->node_of[l].p, P.nodes.p, P.box.p, s->x, s->y, s->z, s->node_of[l + 1].p);
+        // here, beside the head solve, rather than between the level solves
+        if (order && cg_order(s, C))
+            return QZ_FAILURE;
         s->amr_nlev = l + 2;
         if (!check_cuda(cudaGetLastError(), "amr build"))
             return QZ_FAILURE;
@@ -1293,7 +1331,7 @@ int amr_deposit(qz_sim *s)
         if (scan_exclusive(s, flag, slot, n))
             return QZ_FAILURE;
         int t[2];
-        if (!read_at(s, s->amr_tmp.p, {(int)(2 * n - 1), (int)(n - 1)}, t))
+        if (!read_at(s, {slot + n - 1, flag + n - 1}, t))
             return QZ_FAILURE;
         const long m = t[0] + t[1];
         launch(s, QZ_PROF_DEPOSIT, 44.0 * n, k_lvl_keys, dim3(blocks_for(n, 256)), dim3(256), n,
@@ -1457,7 +1495,6 @@ struct CgArgs {
 };
 
 constexpr long long CG_EMPTY = -1LL; // all-ones word: partial not yet published
-constexpr int CG_FILL = 148;         // chunks a level's CG points are cut into (B200's SMs)
 // Interior points a thread in a chunk's update phase (chunks of up to CG_UPT x
 // 512 points), with one block a SM and the registers of one (128 a thread).
 // Measured on the 1M-particle sphere in one run (CG time a step): 2 points a
@@ -2506,19 +2543,54 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     }
     const long max_blocks = (long)per_sm * sms;
     const int nt = CG_MAX_THREADS;
-    // The level's CG points are cut into about CG_FILL chunks (one block a SM),
-    // or 2 CG_FILL when a chunk would exceed the CG_UPT points a thread the
-    // update phase holds: the slowest SM sets every phase's length, so chunks fill
-    // the SMs evenly.  Measured on the 1M-particle sphere with two points a
-    // thread (CG time a step): fixed 1024-point chunks 6.98 ms, CG_FILL 148
-    // 6.86 ms, 74 6.89, 222 7.88, 296 7.60.  CG_FILL is fixed, not the device's
-    // SM count, so the partial sums and the results do not depend on the device.
+    std::vector<int> sor_nodes; // nodes of at most branch_cg_cells cells: red-black SOR
+    for (int q = 0; q < nn; q++)
+        if (!(ov && ov->skip[q]) && allow_sor && L.h[q].ncells <= c.branch_cg_cells &&
+            L.h[q].nintr > 0)
+            sor_nodes.push_back(q);
+    // solver schedule (forward solves only): replay gives every node its recorded count
+    const bool replay = !ov && s->sched_mode == 2;
+    const bool record = !ov && s->sched_mode == 1;
+    std::vector<int> caps;
+    if (replay)
+    {
+        if (!sor_nodes.empty())
+        {
+            set_error("a solver schedule cannot replay red-black SOR nodes");
+            return QZ_FAILURE;
+        }
+        caps.resize(nn);
+        if (!sched_take(s, nn, caps.data()))
+            return QZ_FAILURE;
+    }
+    // Nodes the two-phase kernel would solve go on chip where they fit; the others,
+    // and the other arrangements, keep their vectors in memory.
+    std::vector<char> onchip(nn, 0);
+    std::vector<int> node_cap(nn, 0);
+    for (int q = 0; q < nn; q++)
+    {
+        const AmrNode &N = L.h[q];
+        const bool cg = !(ov && ov->skip[q]) && (!allow_sor || N.ncells > c.branch_cg_cells);
+        onchip[q] = cg && !one && L.cg_ordered && N.nintr > 0 &&
+                    N.nrows <= (long)CG_FILL * CGR_CHUNK_MAX && max_blocks >= CG_FILL;
+        const long size = (long)(N.rd[0] + 1) * (N.rd[1] + 1) * (N.rd[2] + 1);
+        node_cap[q] = replay ? caps[q] : (int)std::min<long>(size, c.max_iter);
+    }
+    // Their chunks: the level's other CG points are cut into about CG_FILL chunks
+    // (one block a SM), or 2 CG_FILL when a chunk would exceed the CG_UPT points a
+    // thread the update phase holds: the slowest SM sets every phase's length, so
+    // chunks fill the SMs evenly.  CG_FILL is fixed, not the device's SM count, so
+    // the partial sums and the results do not depend on the device.
+    auto in_memory = [&](int q) {
+        return !(ov && ov->skip[q]) && (!allow_sor || L.h[q].ncells > c.branch_cg_cells) &&
+               !onchip[q];
+    };
     int chunk = (pipe ? CG2_PPT : 2) * nt;
     if (!pipe)
     {
         long tot = 0;
         for (int q = 0; q < nn; q++)
-            if (!(ov && ov->skip[q]) && (!allow_sor || L.h[q].ncells > c.branch_cg_cells))
+            if (in_memory(q))
                 tot += L.h[q].nintr;
         long target = CG_FILL;
         long cs = (tot + CG_FILL - 1) / CG_FILL;
@@ -2536,7 +2608,7 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
         auto count = [&](long size) {
             long k = 0;
             for (int q = 0; q < nn; q++)
-                if (!(ov && ov->skip[q]) && (!allow_sor || L.h[q].ncells > c.branch_cg_cells))
+                if (in_memory(q))
                     k += (L.h[q].nintr + size - 1) / size;
             return k;
         };
@@ -2548,36 +2620,18 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     L.hchunks.clear();
     std::vector<int> &node_chunk = L.hnode_chunk;
     node_chunk.assign(2L * nn, 0);
-    std::vector<int> sor_nodes; // nodes of at most branch_cg_cells cells: red-black SOR
     for (int q = 0; q < nn; q++)
     {
         node_chunk[2 * q] = (int)L.hchunks.size();
         const AmrNode &N = L.h[q];
-        if (ov && ov->skip[q])
-            ; // no work for this node
-        else if (!allow_sor || N.ncells > c.branch_cg_cells)
+        if (in_memory(q))
             for (int b = N.intr_off; b < N.intr_off + N.nintr; b += chunk)
                 L.hchunks.push_back({q, b, std::min(b + chunk, N.intr_off + N.nintr)});
-        else if (N.nintr > 0)
-            sor_nodes.push_back(q);
         node_chunk[2 * q + 1] = (int)L.hchunks.size();
     }
     L.nchunks = (int)L.hchunks.size();
-    // solver schedule (forward solves only): replay gives every node its recorded count
-    const bool replay = !ov && s->sched_mode == 2;
-    const bool record = !ov && s->sched_mode == 1;
-    std::vector<int> caps;
-    if (replay)
-    {
-        if (!sor_nodes.empty())
-        {
-            set_error("a solver schedule cannot replay red-black SOR nodes");
-            return QZ_FAILURE;
-        }
-        caps.resize(nn);
-        if (!sched_take(s, nn, caps.data()))
-            return QZ_FAILURE;
-    }
+    std::vector<CgrRound> rounds;
+    cgr_plan(L, onchip, node_cap, c.cg_chunk_min, L.hchunks, node_chunk, rounds);
     if (!sor_nodes.empty() && sor_level(s, L, level_index, sor_nodes))
         return QZ_FAILURE;
     pd = CgPending();
@@ -2586,14 +2640,15 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     pd.one = one;
     pd.pipe = pipe;
     pd.nn = nn;
-    if (L.nchunks == 0)
+    if (L.hchunks.empty())
         return QZ_SUCCESS;
     // nint: node_chunk (2 nn) | rfail[0] (nn) | rfail[1] (nn) | status (3) | iterations (nn)
     const long nparts = (one ? 3L : 4L) * L.nchunks * CG_PS;
-    if (!L.chunks.ensure(s->mem, L.nchunks) || !L.chunk_part.ensure(s->mem, nparts) ||
-        !L.nint.ensure(s->mem, 6L * nn + 3) || !L.r.ensure(s->mem, L.grid_total) ||
-        !L.p.ensure(s->mem, L.grid_total) || !L.Ap.ensure(s->mem, L.grid_total) ||
-        !L.apv.ensure(s->mem, L.grid_total) ||
+    const bool mem_cg = L.nchunks > 0; // some nodes' vectors stay in memory
+    if (!L.chunks.ensure(s->mem, (long)L.hchunks.size()) || !L.nint.ensure(s->mem, 6L * nn + 3) ||
+        (mem_cg && (!L.chunk_part.ensure(s->mem, nparts) || !L.r.ensure(s->mem, L.grid_total) ||
+                    !L.p.ensure(s->mem, L.grid_total) || !L.Ap.ensure(s->mem, L.grid_total) ||
+                    !L.apv.ensure(s->mem, L.grid_total))) ||
         (one && !L.cg1.ensure(s->mem, 4 * L.grid_total)))
     {
         set_error("cg buffers");
@@ -2607,11 +2662,36 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     node_chunk[4L * nn + 2] = active;
     for (int q = 0; q < (int)caps.size(); q++)
         node_chunk[5L * nn + 3 + q] = caps[q];
-    if (!check_cuda(cudaMemcpyAsync(L.chunks.p, L.hchunks.data(), L.nchunks * sizeof(AmrChunk),
-                                    cudaMemcpyHostToDevice, s->stream), "chunks") ||
+    if (!check_cuda(cudaMemcpyAsync(L.chunks.p, L.hchunks.data(),
+                                    L.hchunks.size() * sizeof(AmrChunk), cudaMemcpyHostToDevice,
+                                    s->stream), "chunks") ||
         !check_cuda(cudaMemcpyAsync(L.nint.p, node_chunk.data(), (6L * nn + 3) * sizeof(int),
                                     cudaMemcpyHostToDevice, s->stream), "cg ints"))
         return QZ_FAILURE;
+    pd.launched = true;
+    pd.status = L.nint.p + 4 * nn;
+    pd.onchip = onchip;
+    if (!rounds.empty())
+    {
+        CgrSolve v{};
+        v.chunks = L.chunks.p + L.nchunks;
+        // the plan's rounds count from the end of the in-memory chunks
+        for (CgrRound &R : rounds)
+            R.first -= L.nchunks;
+        v.node_chunk = L.nint.p;
+        v.status = L.nint.p + 4 * nn;
+        v.iters = L.nint.p + 4 * nn + 3;
+        v.tol = c.tol;
+        v.tol2 = ov ? ov->tol2 : c.tol2;
+        // replay: decisions by the (never met) r.r threshold only
+        v.method = ov || replay ? 0 : c.check_method;
+        v.thr_node = ov ? ov->thr : nullptr;
+        v.cap_node = replay ? L.nint.p + 5 * nn + 3 : nullptr;
+        if (cgr_launch(s, L, rounds, v))
+            return QZ_FAILURE;
+    }
+    if (!mem_cg)
+        return QZ_SUCCESS;
     // r and both p buffers are zero off the interior points; partials start unpublished
     cudaMemsetAsync(L.r.p, 0, L.grid_total * sizeof(double), s->stream);
     cudaMemsetAsync(L.p.p, 0, L.grid_total * sizeof(double), s->stream);
@@ -2727,8 +2807,6 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
         s->prof_pending.push_back({QZ_PROF_CG, 0.0, eb, ee});
         pd.prof_idx = (int)s->prof_pending.size() - 1;
     }
-    pd.launched = true;
-    pd.status = A.status;
     return QZ_SUCCESS;
 }
 
@@ -2759,7 +2837,8 @@ static int cg_level_collect(qz_sim *s, AmrLevel &L, int level_index, const CgPen
         // the pipelined form reads w, z, s, p, r, pot and writes the six (96 B)
         double pts_it = 0.0;
         for (int q = 0; q < nn; q++)
-            pts_it += (double)L.h[q].nintr * st[3 + q];
+            if (pd.onchip.empty() || !pd.onchip[q])
+                pts_it += (double)L.h[q].nintr * st[3 + q];
         s->prof_pending[pd.prof_idx].bytes = (pipe ? 96.0 : one ? 80.0 : 64.0) * pts_it;
     }
     if (st[1])
@@ -2991,7 +3070,10 @@ int head_cg_solve(qz_sim *s)
     }
     L.h[0].mass = s->head_mass;
     L.h[0].nptcl = (int)s->n;
-    if (!upload_nodes(s, L))
+    const bool order = s->cfg.cg_variant == 0 && !L.cg_ordered;
+    if (order)
+        cg_brick_layout(L);
+    if (!upload_nodes(s, L) || (order && cg_order_list(s, L)))
         return QZ_FAILURE;
     L.d = s->d;
     L.pot = s->pot;
@@ -3025,6 +3107,7 @@ static int node_cg_host(qz_sim *s, int lv, const int rd[3], int nintr, const int
     L.h.assign(1, N);
     L.intr_total = nintr;
     L.grid_total = gt;
+    cg_brick_layout(L);
     if (!L.intr.ensure(s->mem, nintr) || !L.gpot.ensure(s->mem, gt) ||
         !L.gpot_old.ensure(s->mem, gt) || !L.gd.ensure(s->mem, gt) || !upload_nodes(s, L))
     {
@@ -3042,6 +3125,8 @@ static int node_cg_host(qz_sim *s, int lv, const int rd[3], int nintr, const int
                                     cudaMemcpyHostToDevice, s->stream), "node pot_old") ||
         !check_cuda(cudaMemcpyAsync(L.d, d, gt * sizeof(double), cudaMemcpyHostToDevice,
                                     s->stream), "node density"))
+        return QZ_FAILURE;
+    if (s->cfg.cg_variant == 0 && cg_order_list(s, L))
         return QZ_FAILURE;
     const long long it0 = s->stats.cg_iterations;
     const int rc = cg_level(s, L, 0, false);

@@ -208,6 +208,9 @@ struct AmrNode {
     int nptcl;       // particles in the node (no_ptcl_full_node)
     int contact;     // touches the simulation boundary (sim_bdry_contact)
     double mass;     // node_mass
+    int brick_off;   // first brick of the node in the level's 4^3 bricks (conjugate-gradient order)
+    int bbits[3];    // bits of its brick coordinates
+    int row_off, nrows; // its rows in the level's conjugate-gradient order (host copy)
 };
 
 struct AmrChunk {
@@ -297,6 +300,13 @@ struct AmrLevel {
     DBuf<int> mass_range;    // per node: segment range
     DBuf<int> sor;           // red-black SOR nodes of the level and their iteration counts
     int nchunks = 0;
+    // on-chip conjugate gradient: rows of four points in its order (grid index of the
+    // first point, lanes that hold one), row that starts at a grid point (or -1)
+    DBuf<int2> row;
+    DBuf<int> pos;
+    long brick_total = 0;
+    int row_total = 0;
+    bool cg_ordered = false; // row and pos are this tree's
     int h_active = 0; // host copy of the unconverged-node count at the start of a solve
     std::vector<AmrChunk> hchunks;
     std::vector<int> hnode_chunk; // node chunk ranges and flags uploaded with the chunks
@@ -417,6 +427,14 @@ struct qz_sim {
     qz::DBuf<int> zone_cells;          // per zone: cells
     qz::DBuf<int> gather_idx;          // small gathers of scan values
     qz::DBuf<double> seg_mass;         // per deposit segment: mass
+    // on-chip conjugate gradient: exchanged words (halo values, partial sums) and the
+    // next launch's first tag, ghost lists, brick scratch; cgr_ghosts (tests) caps the
+    // ghost rows kept in shared memory
+    qz::DBuf<unsigned long long> cgr_halo, cgr_sums, cgr_list, brick_mask;
+    qz::DBuf<double> cgr_spill;
+    qz::DBuf<int> brick_base;
+    long cgr_tag = 0;
+    int cgr_ghosts = 0;
     int *h_small = nullptr;            // pinned read-back buffer
     long h_small_cap = 0;
 
@@ -550,7 +568,8 @@ struct CgPending {
     bool record = false, replay = false, one = false, pipe = false;
     int nn = 0;
     const int *status = nullptr; // status (3) then iterations (nn)
-    int prof_idx = -1;           // the launch's profiler record, or -1
+    int prof_idx = -1;           // the in-memory launch's profiler record, or -1
+    std::vector<char> onchip;    // nodes solved on chip (their launches book their own bytes)
 };
 bool amr_potential_queues(const qz_sim *s);
 int amr_potential_issue(qz_sim *s, std::vector<CgPending> &pend);

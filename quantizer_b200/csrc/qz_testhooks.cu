@@ -127,3 +127,11 @@ int qz_test_wait_gives_up(qz_sim *s, int which, int *out2)
 }
 
 } // extern "C"
+
+extern "C" QZ_API int qz_test_cg_ghosts(qz_sim *s, int rows)
+{
+    if (!s || rows < 0)
+        return QZ_FAILURE;
+    s->cgr_ghosts = rows;
+    return QZ_SUCCESS;
+}
