@@ -20,7 +20,7 @@ LIBDIR = os.path.join(HERE, "lib")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 CUDA_SOURCES = ["qz_capi.cu", "qz_particles.cu", "qz_poisson.cu", "qz_sort.cu", "qz_amr.cu",
-                "qz_cg_resident.cu", "qz_noalloc.cu", "qz_observe.cu",
+                "qz_cg_resident.cu", "qz_direct.cu", "qz_noalloc.cu", "qz_observe.cu",
                 "qz_ensemble.cu", "qz_adjoint.cu", "qz_snapshot.cu", "qz_testhooks.cu",
                 "qz_node_mg.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

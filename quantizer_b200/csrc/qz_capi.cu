@@ -128,6 +128,7 @@ static bool build_levels(qz_sim *s, int n0)
     // persistent cycles: per-block partials of the in-launch convergence test, its result
     if (!s->mg_part && !dmalloc(&s->mg_part, 2 * QZ_CG_PART_MAX + 8, "mg partials"))
         return false;
+    cudaMemset(s->mg_part, 0, (2 * QZ_CG_PART_MAX + 8) * sizeof(double));
     for (auto &l : s->levels)
     {
         size_t pts = (size_t)l.n * l.n * l.n;
@@ -197,6 +198,8 @@ static void free_levels(qz_sim *s)
     dfree(s->ef);
     dfree(s->ef_alt);
     dfree(s->fine_alt_buf);
+    dfree(s->direct_tab);
+    s->direct_tab = nullptr;
     s->rf = s->ef = s->ef_alt = nullptr;
     s->fine_alt_buf = nullptr;
 }
@@ -787,10 +790,10 @@ namespace qz {
 // 10 points 9.57, 12 points 9.53, 16 points 9.95.
 constexpr int OVERLAP_PPT = 12;
 
-// Outcomes a step reads at its end: the head launch (when it ran on the second
-// stream) and the queued level solves.
+// Outcomes a step reads at its end: the head launch (when it was queued) and the queued level solves.
 struct StepPending {
     bool head = false;
+    cudaStream_t head_stream = nullptr; // where the head launch is queued
     bool levels = false;
     std::vector<CgPending> pend;
 };
@@ -800,7 +803,7 @@ struct StepPending {
 static int step_finish(qz_sim *s, StepPending &sp)
 {
     int rc = QZ_SUCCESS;
-    if (sp.head && potential_head_finish(s, s->head_stream))
+    if (sp.head && potential_head_finish(s, sp.head_stream))
         rc = QZ_FAILURE;
     if (rc == QZ_SUCCESS && sp.levels && amr_potential_collect(s, sp.pend))
         rc = QZ_FAILURE;
@@ -810,6 +813,16 @@ static int step_finish(qz_sim *s, StepPending &sp)
 
 static int tree_density_potential(qz_sim *s, StepPending &sp)
 {
+    if (!amr_on(s) && head_one_launch(s))
+    {
+        // head only: the gradient, gather and kick are queued behind the head solve
+        bool issued = false;
+        sp.head_stream = s->stream;
+        if (deposit_head(s) || potential_head_issue(s, s->stream, &issued))
+            return QZ_FAILURE;
+        sp.head = issued;
+        return QZ_SUCCESS;
+    }
     if (!amr_on(s) || !s->cfg.tree_overlap || s->no_overlap || !head_one_launch(s))
         return (qz_tree_adaptation(s) || qz_grid_density(s) || qz_potential(s)) ? QZ_FAILURE
                                                                                 : QZ_SUCCESS;
@@ -846,6 +859,7 @@ static int tree_density_potential(qz_sim *s, StepPending &sp)
     // last level on the stream; the outcomes (head, then levels) are read at
     // the end of the step (step_finish)
     sp.head = true;
+    sp.head_stream = s->head_stream;
     if (ok && amr_potential_queues(s))
     {
         sp.levels = true;

@@ -343,6 +343,7 @@ struct qz_sim {
     cudaStream_t head_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_head = nullptr;
     bool no_overlap = false; // set by qz_ensemble_step: members stay on one stream
+    bool mg_after_direct = false; // the multigrid launch follows a direct solve
     int mg_ppt_floor = 0;    // fewest finest-level points a thread of the head launch takes
     unsigned *gbar = nullptr;  // grid barrier words of the cooperative launches (4)
     long n = 0, cap = 0;
@@ -359,6 +360,7 @@ struct qz_sim {
     qz::Grid<double> fine_phi{}, fine_rho{}; // level-0 views (head solve grid)
     qz::Grid<double> fine_alt{};             // level-0 red-black ping-pong partner
     double *fine_alt_buf = nullptr;
+    double *direct_tab = nullptr; // direct head solve: twiddles and eigenvalues (qz_direct.cu)
     float *ef_alt = nullptr;
 
     // deposit scratch
@@ -553,6 +555,8 @@ int kick_drift(qz_sim *s, double dt);
 int kick(qz_sim *s, double dt);
 
 int potential_head(qz_sim *s);
+int direct_correct(qz_sim *s, double *phi, double *rho); // qz_direct.cu
+int direct_head(qz_sim *s);
 int amr_init(qz_sim *s);
 void amr_free(qz_sim *s);
 int amr_build(qz_sim *s);

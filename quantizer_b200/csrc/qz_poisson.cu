@@ -803,6 +803,10 @@ template <typename T> struct MgArgs {
     // the launch is one thread-block cluster (at most MG_CLUSTER_MAX blocks):
     // its grid-wide barrier is the hardware cluster barrier
     int cluster;
+    // a direct solve ran before: nothing to do when outst[2] says that it passed the test;
+    // else the red-black partner grid of the fine level takes its boundary first
+    int direct;
+    Grid<double> partner;
 };
 
 // Work item t = a + n0 (b + n1 c) of a grid-stride loop (t = tid, tid + stride,
@@ -1586,6 +1590,9 @@ __global__ void __launch_bounds__(MG_THREADS, 2) k_mg_cycles(const __grid_consta
     extern __shared__ __align__(16) unsigned char mg_dyn[];
     __shared__ int sh_ok;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
+    // after a direct solve that passed the test there is nothing to do
+    if (A.direct && __ldcg(&A.outst[2]))
+        return;
     // every block reaches the same barriers in the same order (all decisions
     // come from values every block computes alike), so the cluster barrier,
     // which has no time limit, is met as surely as the bounded grid barrier
@@ -1595,6 +1602,20 @@ __global__ void __launch_bounds__(MG_THREADS, 2) k_mg_cycles(const __grid_consta
         else
             gbar_sync(A.bar, &sh_ok);
     };
+    if (A.direct)
+    {
+        // the partner grid takes the fine grid's boundary values (it was the transforms'
+        // work space); pot_old is pot already
+        const Grid<double> &P = A.fphi;
+        const unsigned n = (unsigned)P.n, n3 = n * n * n;
+        for (unsigned t = gtid; t < n3; t += gn)
+        {
+            const int i = (int)(t % n), j = (int)(t / n % n), k = (int)(t / (n * n));
+            A.partner.p[A.partner.off + i + j * A.partner.sy + k * A.partner.sz] =
+                P.p[P.off + i + j * P.sy + k * P.sz];
+        }
+        gsync();
+    }
     for (int it = 0; it < A.iters; it++)
     {
         if constexpr (std::is_same<T, double>::value)
@@ -1864,6 +1885,8 @@ static int mg_launch(qz_sim *s, int iters, bool check = false, bool defer = fals
     A.fphi = s->fine_phi;
     A.frho = s->fine_rho;
     A.bar = GridBar{s->gbar, s->flags};
+    A.direct = s->mg_after_direct ? 1 : 0;
+    A.partner = s->fine_alt;
     cudaMemsetAsync(s->gbar, 0, 4 * sizeof(unsigned), s->stream);
     A.check = check ? 1 : 0;
     A.every = A.mixed ? 1 : (c.check_every > 0 ? c.check_every : 1);
@@ -2306,16 +2329,32 @@ static int resid_norms(qz_sim *s, const double *lam, const double *f, double *sc
     return QZ_SUCCESS;
 }
 
+// The direct solve (qz_direct.cu) may stand in for the head's cycles: red-black V-cycles,
+// whose order of updates nothing prescribes, with an iteration cap that is not itself
+// the point (a cap near what the cycles need, 10 to 15, decides between success and
+// failure).
+constexpr int DIRECT_MIN_CAP = 100;
+
+static bool direct_allowed(const qz_sim *s)
+{
+    const qz_config &c = s->cfg;
+    return c.smoother == 0 && c.gs_order == QZ_GS_REDBLACK && c.cycle == 0 && !s->fused_rb &&
+           c.max_iter >= DIRECT_MIN_CAP && s->fine_alt_buf;
+}
+
 // Solves Lap_h lam = f on the head interior with lam = 0 on the solve grid's
-// boundary, by FP64 multigrid cycles of the configured kind (the operator of
-// the head solve is symmetric, so this is also its adjoint), from the initial
-// guess in lam, until |r| <= rtol |f| (checked every 2 cycles).  scratch holds
-// 2 * red_blocks + 2 doubles; host 2 pinned doubles.  *cycles: cycles run.
+// boundary until |r| <= rtol |f|: directly where that is allowed, then, while the
+// goal is not met, by FP64 multigrid cycles of the configured kind (the operator of
+// the head solve is symmetric, so this is also its adjoint; checked every 2
+// cycles).  scratch holds 2 * red_blocks + 2 doubles; host 2 pinned doubles.
+// *cycles: cycles run.
 int solve_zero_bc(qz_sim *s, double *lam, double *f, double rtol, double *scratch,
                   double *host, int *cycles)
 {
     const qz_config &c = s->cfg;
     *cycles = 0;
+    if (direct_allowed(s) && direct_correct(s, lam, f))
+        return QZ_FAILURE;
     if (resid_norms(s, lam, f, scratch, host))
         return QZ_FAILURE;
     if (host[1] == 0.0)
@@ -2410,9 +2449,16 @@ int poisson_error_head(qz_sim *s, int *converged)
     return QZ_SUCCESS;
 }
 
-// The head solve is one persistent launch with the convergence test inside it
-// (multigrid cycles of the red-black V-cycle, FP64 or the mixed form, no
-// replayed schedule).
+// The head solve starts with the direct solve, except under a solver schedule, whose
+// counts are cycles.
+static bool head_direct(const qz_sim *s)
+{
+    return s->cfg.head_pot_method != 1 && s->sched_mode == 0 && direct_allowed(s);
+}
+
+// The head solve is queued without a host wait: the direct solve and, where its result
+// does not pass the test, one persistent launch of cycles with the test inside it
+// (red-black V-cycles, FP64 or the mixed form, no replayed schedule).
 bool head_one_launch(const qz_sim *s)
 {
     return s->cfg.head_pot_method != 1 && s->sched_mode != 2 && mg_persistent(s);
@@ -2448,13 +2494,27 @@ int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued)
     const qz_config &c = s->cfg;
     cudaStream_t keep = s->stream;
     s->stream = st;
-    cudaMemcpyAsync(s->pot_old, s->pot, s->gpts * sizeof(double), cudaMemcpyDeviceToDevice,
-                    s->stream);
-    sync_fine_alt(s);
+    const bool direct = head_direct(s);
+    if (direct)
+    {
+        if (direct_head(s))
+        {
+            s->stream = keep;
+            return QZ_FAILURE;
+        }
+    }
+    else
+    {
+        cudaMemcpyAsync(s->pot_old, s->pot, s->gpts * sizeof(double), cudaMemcpyDeviceToDevice,
+                        s->stream);
+        sync_fine_alt(s);
+    }
+    s->mg_after_direct = direct;
     // the mixed form tests after every defect-correction iteration (its FP64
     // residual is computed anyway); the FP64 form keeps the reference's cadence
     const int rc = c.precision == QZ_PREC_MIXED ? mg_launch<float>(s, c.max_iter, true, true)
                                                 : mg_launch<double>(s, c.max_iter, true, true);
+    s->mg_after_direct = false;
     s->stream = keep;
     *issued = rc == QZ_SUCCESS;
     return rc;
@@ -2496,13 +2556,25 @@ int potential_head(qz_sim *s)
             return QZ_FAILURE;
         return potential_head_finish(s, s->stream);
     }
+    int iter = 0;
+    bool check = false;
+    if (head_direct(s))
+    {
+        int ok = 0;
+        const int *outst = reinterpret_cast<const int *>(s->mg_part + 2 * QZ_CG_PART_MAX);
+        if (direct_head(s) ||
+            !check_cuda(cudaMemcpyAsync(&ok, outst + 2, sizeof ok, cudaMemcpyDeviceToHost,
+                                        s->stream), "direct solve result") ||
+            !check_cuda(cudaStreamSynchronize(s->stream), "direct solve result"))
+            return QZ_FAILURE;
+        if (ok)
+            return head_tail(s, 0, true);
+    }
     cudaMemcpyAsync(s->pot_old, s->pot, s->gpts * sizeof(double), cudaMemcpyDeviceToDevice,
                     s->stream);
     if (c.head_pot_method == 1)
         return head_cg_solve(s);
     sync_fine_alt(s);
-    int iter = 0;
-    bool check = false;
     if (s->sched_mode == 2)
     {
         // replay: exactly the recorded number of cycles, no convergence test
