@@ -151,10 +151,9 @@ __device__ __forceinline__ void adj_cic_add(int i, double scale, const double *_
     }
 }
 
-// One warp per occupied cell of at most SEG_LONG particles (longer cells are
-// listed for k_adj_seg_long): for each of the 8 corners the sums of w * abar
-// over the cell's particles, three components.  cs: segment * 24 + component *
-// 8 + corner.
+// For every occupied cell of at most SEG_LONG particles (longer cells are listed for
+// k_adj_seg_long) and each of its 8 corners the sums of w * abar over the cell's particles,
+// three components.  cs: segment * 24 + component * 8 + corner.
 __global__ void k_adj_seg_reduce(int L, const int *__restrict__ perm,
                                  const int *__restrict__ seg_start, int *__restrict__ flags,
                                  int *__restrict__ long_list, const double *__restrict__ x,
@@ -162,44 +161,11 @@ __global__ void k_adj_seg_reduce(int L, const int *__restrict__ perm,
                                  const double *__restrict__ abx, const double *__restrict__ aby,
                                  const double *__restrict__ abz, double *__restrict__ cs)
 {
-    const int lane = threadIdx.x & 31;
-    const long warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    const int nseg = flags[F_NSEG];
     const double scale = (double)(1 << L);
-    for (long sg = warp0; sg < nseg; sg += nwarps)
-    {
-        const int b = seg_start[sg], e = seg_start[sg + 1];
-        if (e - b > SEG_LONG)
-        {
-            if (lane == 0)
-                long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sg;
-            continue;
-        }
-        double acc[24];
-#pragma unroll
-        for (int c = 0; c < 24; c++)
-            acc[c] = 0.0;
-        for (int q = b + lane; q < e; q += 32)
-            adj_cic_add(perm[q], scale, x, y, z, abx, aby, abz, acc);
-#pragma unroll
-        for (int c = 0; c < 24; c++)
-        {
-            double v = acc[c];
-            for (int o = 16; o > 0; o >>= 1)
-                v += __shfl_xor_sync(0xffffffffu, v, o);
-            acc[c] = v;
-        }
-        if (lane < 24)
-        {
-            double v = acc[0];
-#pragma unroll
-            for (int c = 1; c < 24; c++)
-                if (lane == c)
-                    v = acc[c];
-            cs[sg * 24 + lane] = v;
-        }
-    }
+    seg_sums<3, false>(
+        flags[F_NSEG], perm, seg_start, flags, long_list,
+        [&](int i, double (&acc)[24]) { adj_cic_add(i, scale, x, y, z, abx, aby, abz, acc); },
+        [&](long sg, int c, double v) { cs[sg * 24 + c] = v; });
 }
 
 // One block per listed cell of more than SEG_LONG particles: thread t adds
@@ -687,21 +653,40 @@ __global__ void k_adj_lvl_negdiv(long total, int nn, const AmrNode *__restrict__
     out[g] = v * o2h + phic[g];
 }
 
-// per node: sum of rhs^2 over its interior list (one block a node, fixed order)
+// per node: sum of rhs^2 over its interior list, in a fixed order: block (node, j) adds
+// the j-th of ADJ_NORM_PARTS slices, the second kernel the slices (one block a node
+// took 290 us for 100,000 points, mostly waiting for its loads; now 8)
+constexpr int ADJ_NORM_PARTS = 64;
+
 __global__ void k_adj_node_norm(const AmrNode *__restrict__ nodes, const int *__restrict__ intr,
-                                const double *__restrict__ rhs, double *__restrict__ out)
+                                const double *__restrict__ rhs, double *__restrict__ part)
 {
     __shared__ double sh[32];
     const AmrNode N = nodes[blockIdx.x];
+    const int len = (N.nintr + ADJ_NORM_PARTS - 1) / ADJ_NORM_PARTS;
+    const int b = blockIdx.y * len, e1 = min(N.nintr, b + len);
     double acc = 0.0;
-    for (int e = threadIdx.x; e < N.nintr; e += blockDim.x)
+#pragma unroll 4
+    for (int e = b + threadIdx.x; e < e1; e += blockDim.x)
     {
         const double v = rhs[intr[N.intr_off + e]];
         acc += v * v;
     }
     acc = adj_block_sum(acc, sh);
     if (threadIdx.x == 0)
-        out[blockIdx.x] = acc;
+        part[blockIdx.x * ADJ_NORM_PARTS + blockIdx.y] = acc;
+}
+
+__global__ void k_adj_node_norm_sum(int nn, const double *__restrict__ part,
+                                    double *__restrict__ out)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nn)
+        return;
+    double t = 0.0;
+    for (int j = 0; j < ADJ_NORM_PARTS; j++)
+        t += part[q * ADJ_NORM_PARTS + j];
+    out[q] = t;
 }
 
 // phi-bar of a boundary point after the solve: its own minus the solve's
@@ -1041,7 +1026,7 @@ static int adj_alloc_levels(qz_sim *s)
             cudaMemsetAsync(A.llam[l].p, 0, A.llam[l].cap * sizeof(double), s->stream);
         nnmax = std::max(nnmax, (long)L.nnodes);
     }
-    return A.nrm.ensure(s->mem, nnmax) ? QZ_SUCCESS : QZ_FAILURE;
+    return A.nrm.ensure(s->mem, (1 + ADJ_NORM_PARTS) * nnmax) ? QZ_SUCCESS : QZ_FAILURE;
 }
 
 // a-bar deposited on the grid of level l >= 1 from the particles whose finest
@@ -1088,7 +1073,6 @@ static int adj_level_deposit(qz_sim *s, int l, const double *x, const double *y,
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
     const long blocks = std::min((m * 32 + 255) / 256, (long)sms * 16);
-    cudaMemsetAsync(s->flags + F_NLONG, 0, sizeof(int), s->stream);
     launch(s, QZ_PROF_DEPOSIT, 56.0 * m, k_adj_seg_reduce, dim3((int)blocks), dim3(256),
            L.h[0].lv, perm, s->seg_start, s->flags, s->long_seg, x, y, z, ab, ab + n, ab + 2 * n,
            A.cs.p);
@@ -1148,7 +1132,6 @@ static int force_vjp(qz_sim *s, const double *x, const double *y, const double *
     const long blocks = std::min((n * 32 + 255) / 256, (long)sms * 16);
     if (!A.cs.ensure(s->mem, 24 * n + 24))
         return QZ_FAILURE;
-    cudaMemsetAsync(s->flags + F_NLONG, 0, sizeof(int), s->stream);
     launch(s, QZ_PROF_DEPOSIT, 56.0 * n, k_adj_seg_reduce, dim3((int)blocks), dim3(256), L, perm,
            s->seg_start, s->flags, s->long_seg, x, y, z, abh, abh + n, abh + 2 * n, A.cs.p);
     launch(s, QZ_PROF_DEPOSIT, 0.0, k_adj_seg_long, dim3(2 * sms), dim3(ADJ_SEG_LONG_THREADS), L, perm,
@@ -1208,8 +1191,12 @@ static int force_vjp(qz_sim *s, const double *x, const double *y, const double *
                    dim3(256), gt, Lv.nnodes, Lv.nodes.p, A.lmask[l].p, A0, A1, A2, A.lphic[l].p,
                    A.lphib[l].p);
             // node thresholds from the rhs norms; nodes with a zero rhs keep lam = 0
-            launch(s, QZ_PROF_OTHER, 8.0 * Lv.intr_total, k_adj_node_norm, dim3(Lv.nnodes),
-                   dim3(256), Lv.nodes.p, Lv.intr.p, A.lphib[l].p, A.nrm.p);
+            launch(s, QZ_PROF_OTHER, 8.0 * Lv.intr_total, k_adj_node_norm,
+                   dim3(Lv.nnodes, ADJ_NORM_PARTS), dim3(256), Lv.nodes.p, Lv.intr.p, A.lphib[l].p,
+                   A.nrm.p + Lv.nnodes);
+            launch(s, QZ_PROF_OTHER, 8.0 * ADJ_NORM_PARTS * Lv.nnodes, k_adj_node_norm_sum,
+                   dim3(blocks_for(Lv.nnodes, 128)), dim3(128), Lv.nnodes, A.nrm.p + Lv.nnodes,
+                   A.nrm.p);
             std::vector<double> nrm(Lv.nnodes);
             if (!check_cuda(cudaMemcpyAsync(nrm.data(), A.nrm.p, Lv.nnodes * sizeof(double),
                                             cudaMemcpyDeviceToHost, s->stream), "node norms") ||

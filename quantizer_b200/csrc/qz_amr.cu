@@ -1019,8 +1019,8 @@ __device__ __forceinline__ void lvl_cic_add(int i, double H, double ooh, double 
     acc[8] += m[i];
 }
 
-// One warp per occupied cell of at most SEG_LONG particles (longer cells are
-// listed for k_lvl_seg_long): the corner sums and the cell's mass.
+// The corner sums and the mass of every occupied cell of at most SEG_LONG particles
+// (longer cells are listed for k_lvl_seg_long).
 __global__ void k_lvl_seg_reduce(int lv, double coeff, const int *__restrict__ perm,
                                  const int *__restrict__ seg_start, int *__restrict__ flags,
                                  int *__restrict__ long_list, const double *__restrict__ x,
@@ -1028,135 +1028,17 @@ __global__ void k_lvl_seg_reduce(int lv, double coeff, const int *__restrict__ p
                                  const double *__restrict__ m, double *__restrict__ cs,
                                  double *__restrict__ smass)
 {
-    const int lane = threadIdx.x & 31;
-    const long warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    const int nseg = flags[F_NSEG];
     const double H = 1.0 / (1 << lv);
     const double ooh = (double)(1 << lv);
-    // A warp takes four consecutive cells.  When each holds at most 8 particles,
-    // lanes 8g..8g+7 sum cell g (one particle a lane): the xor tree over those 8
-    // lanes is the tree the whole warp would apply to them (the other lanes hold
-    // zeros, which add exactly), so the sums are bit for bit those of one warp a
-    // cell.
-    for (long s4 = warp0 * 4; s4 < nseg; s4 += nwarps * 4)
-    {
-        const int g = lane >> 3, gl = lane & 7;
-        const long sgg = s4 + g;
-        int bg = 0, eg = 0;
-        if (sgg < nseg)
-        {
-            bg = seg_start[sgg];
-            eg = seg_start[sgg + 1];
-        }
-        if (__all_sync(0xffffffffu, eg - bg <= 8))
-        {
-            double acc[9];
-#pragma unroll
-            for (int c = 0; c < 9; c++)
-                acc[c] = 0.0;
-            if (gl < eg - bg)
-                lvl_cic_add(perm[bg + gl], H, ooh, coeff, x, y, z, m, acc);
-#pragma unroll
-            for (int c = 0; c < 9; c++)
-            {
-                double v = acc[c];
-                for (int o = 4; o > 0; o >>= 1)
-                    v += __shfl_xor_sync(0xffffffffu, v, o);
-                acc[c] = v;
-            }
-            if (sgg < nseg)
-            {
-                double v = acc[0];
-#pragma unroll
-                for (int c = 1; c < 8; c++)
-                    if (gl == c)
-                        v = acc[c];
-                cs[sgg * 8 + gl] = v;
-                if (gl == 0)
-                    smass[sgg] = acc[8];
-            }
-            continue;
-        }
-        // else pairs of cells of at most 16 particles, 16 lanes a cell (again the
-        // warp's tree), and one warp a cell for the others
-        for (int h = 0; h < 2; h++)
-        {
-            const long p0 = s4 + 2 * h;
-            const int gh = lane >> 4, hl = lane & 15;
-            const long sgp = p0 + gh;
-            int bp = 0, ep = 0;
-            if (sgp < nseg)
-            {
-                bp = seg_start[sgp];
-                ep = seg_start[sgp + 1];
-            }
-            if (__all_sync(0xffffffffu, ep - bp <= 16))
-            {
-                double acc[9];
-#pragma unroll
-                for (int c = 0; c < 9; c++)
-                    acc[c] = 0.0;
-                if (hl < ep - bp)
-                    lvl_cic_add(perm[bp + hl], H, ooh, coeff, x, y, z, m, acc);
-#pragma unroll
-                for (int c = 0; c < 9; c++)
-                {
-                    double v = acc[c];
-                    for (int o = 8; o > 0; o >>= 1)
-                        v += __shfl_xor_sync(0xffffffffu, v, o);
-                    acc[c] = v;
-                }
-                if (sgp < nseg && hl < 8)
-                {
-                    double v = acc[0];
-#pragma unroll
-                    for (int c = 1; c < 8; c++)
-                        if (hl == c)
-                            v = acc[c];
-                    cs[sgp * 8 + hl] = v;
-                    if (hl == 0)
-                        smass[sgp] = acc[8];
-                }
-                continue;
-            }
-            for (long sg = p0; sg < p0 + 2 && sg < nseg; sg++)
-            {
-                const int b = seg_start[sg], e = seg_start[sg + 1];
-                if (e - b > SEG_LONG)
-                {
-                    if (lane == 0)
-                        long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sg;
-                    continue;
-                }
-                double acc[9];
-#pragma unroll
-                for (int c = 0; c < 9; c++)
-                    acc[c] = 0.0;
-                for (int q = b + lane; q < e; q += 32)
-                    lvl_cic_add(perm[q], H, ooh, coeff, x, y, z, m, acc);
-#pragma unroll
-                for (int c = 0; c < 9; c++)
-                {
-                    double v = acc[c];
-                    for (int o = 16; o > 0; o >>= 1)
-                        v += __shfl_xor_sync(0xffffffffu, v, o);
-                    acc[c] = v;
-                }
-                if (lane < 8)
-                {
-                    double v = acc[0];
-#pragma unroll
-                    for (int c = 1; c < 8; c++)
-                        if (lane == c)
-                            v = acc[c];
-                    cs[sg * 8 + lane] = v;
-                }
-                if (lane == 0)
-                    smass[sg] = acc[8];
-            }
-        }
-    }
+    seg_sums<1, true>(
+        flags[F_NSEG], perm, seg_start, flags, long_list,
+        [&](int i, double (&acc)[9]) { lvl_cic_add(i, H, ooh, coeff, x, y, z, m, acc); },
+        [&](long sg, int c, double v) {
+            if (c < 8)
+                cs[sg * 8 + c] = v;
+            else
+                smass[sg] = v;
+        });
 }
 
 // One block per listed cell of more than SEG_LONG particles (as k_seg_long).
@@ -1353,7 +1235,6 @@ int amr_deposit(qz_sim *s)
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
         long blocks = std::min((m * 32 + 255) / 256 + 1, (long)sms * 16);
-        cudaMemsetAsync(s->flags + F_NLONG, 0, sizeof(int), s->stream);
         launch(s, QZ_PROF_DEPOSIT, 40.0 * m, k_lvl_seg_reduce, dim3((int)blocks), dim3(256),
                L.h[0].lv, coeff, perm, s->seg_start, s->flags, s->long_seg, s->x, s->y, s->z,
                s->m, s->cell_sums, s->seg_mass.p);

@@ -399,7 +399,7 @@ int qz_destroy(qz_sim *s)
     s->ev_pool.clear();
     void *ptrs[] = {s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az, s->m,
                     s->pot, s->pot_old, s->d, s->gax, s->gay, s->gaz, s->sort.k0, s->sort.k1,
-                    s->sort.v0, s->sort.v1, s->sort.hist, s->seg_head, s->seg_id, s->seg_start,
+                    s->sort.v0, s->sort.v1, s->sort.hist, s->seg_start,
                     s->seg_cell, s->cell_seg, s->cell_sums, s->red, s->flags, s->d_ts,
                     s->gbar, s->long_seg};
     for (void *p : ptrs)
@@ -530,8 +530,7 @@ int qz_create(const qz_config *cfg, long n_capacity, qz_sim **out)
     ok = ok && dmalloc(&s->sort.k0, cap, "keys") && dmalloc(&s->sort.k1, cap, "keys") &&
          dmalloc(&s->sort.v0, cap, "vals") && dmalloc(&s->sort.v1, cap, "vals") &&
          dmalloc(&s->sort.hist, 256 * std::max(tiles, 4L), "hist");
-    ok = ok && dmalloc(&s->seg_head, cap, "seg") && dmalloc(&s->seg_id, cap, "seg") &&
-         dmalloc(&s->seg_start, cap + 1, "seg") && dmalloc(&s->seg_cell, cap, "seg") &&
+    ok = ok && dmalloc(&s->seg_start, cap + 1, "seg") && dmalloc(&s->seg_cell, cap, "seg") &&
          dmalloc(&s->cell_seg, B * B * B, "cell_seg") && dmalloc(&s->cell_sums, 8 * cap, "cs") &&
          dmalloc(&s->long_seg, cap / SEG_LONG + 2, "long segments");
     s->red_blocks = 296;

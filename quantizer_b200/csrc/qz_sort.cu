@@ -5,8 +5,8 @@
 // original element order; the scan's tile numbers follow the blocks' arrival,
 // but its results are integer sums and do not depend on it).
 //
-// Tile = 8 warps x 8 iterations x 32 lanes = 2048 keys.  Warp w of tile t
-// owns keys [t*2048 + w*256, +256); iteration r covers 32 consecutive keys in
+// Tile = 16 warps x 8 iterations x 32 lanes = 4096 keys.  Warp w of tile t
+// owns keys [t*4096 + w*256, +256); iteration r covers 32 consecutive keys in
 // lane order, so (warp, iteration, lane) order is the input order and the
 // scatter is stable.  One pass per 8-bit digit, each a single launch
 // (Adinets and Merrill's one-sweep arrangement, 2022): the digit counts of all
@@ -19,9 +19,10 @@
 
 namespace qz {
 
-constexpr int RS_WARPS = 8;
+constexpr int RS_WARPS = 16;
 constexpr int RS_ITEMS = 8;
-constexpr int RS_TILE = RS_WARPS * RS_ITEMS * 32; // 2048
+constexpr int RS_TILE = RS_WARPS * RS_ITEMS * 32; // 4096
+constexpr int RS_BACK = 8; // status words of a look-back in flight together
 constexpr int RS_RADIX = 256;
 
 // ---- exclusive scan -------------------------------------------------------------------
@@ -228,12 +229,17 @@ __global__ void k_rs_hist(const unsigned *__restrict__ keys, long n, int passes,
 }
 
 // One pass on the digit at `shift`.  A block takes the next tile number from
-// the counter (arrival order, as the scan), counts its keys per warp and digit,
-// publishes its per-digit counts in the status words of its tile (flag | epoch
+// the counter (arrival order, as the scan), loads its keys and values, ranks every
+// key among the equal digits before it in its warp (match masks, a running count a
+// digit), publishes the tile's per-digit counts in its status words (flag | epoch
 // | value, as the scan's), and thread d adds the counts of digit d in the tiles
-// before it, walking back to the first inclusive prefix; the digit's output
-// base is the exclusive scan of the pass's global counts plus that prefix.  The
-// scatter is the stable warp-ordered one.
+// before it, RS_BACK of them a trip, back to the first inclusive prefix; the digit's
+// output base is the exclusive scan of the pass's global counts plus that prefix.
+// The pairs are put in order in shared memory first, so that a digit's run leaves in
+// consecutive stores.  A pass is a chain of trips (tile number, keys, look-back,
+// stores) rather than bytes: with 2048-key tiles, keys loaded twice one iteration at a
+// time, one predecessor a trip and scattered stores it took 14 us at 10,000 keys and
+// 31 at 1M; now 7 and 17.
 __global__ void __launch_bounds__(RS_WARPS * 32)
     k_rs_onesweep(const unsigned *__restrict__ kin, const int *__restrict__ vin,
                   unsigned *__restrict__ kout, int *__restrict__ vout, long n, int shift,
@@ -241,87 +247,131 @@ __global__ void __launch_bounds__(RS_WARPS * 32)
                   unsigned long long *__restrict__ ctr, unsigned long long base, unsigned epoch,
                   int *__restrict__ flags)
 {
-    static_assert(RS_WARPS * 32 == RS_RADIX, "one thread a digit");
-    __shared__ int woff[RS_WARPS][RS_RADIX];
-    __shared__ int bbase[RS_RADIX];
+    static_assert(RS_WARPS * 32 >= RS_RADIX, "a thread a digit");
+    __shared__ int woff[RS_WARPS][RS_RADIX]; // then the ordered keys
+    static_assert(RS_TILE == RS_WARPS * RS_RADIX, "the keys take the counts' place");
+    unsigned *skey = reinterpret_cast<unsigned *>(&woff[0][0]);
+    __shared__ int sval[RS_TILE];
+    __shared__ int goff[RS_RADIX]; // output place of a digit's first key less its place in the tile
+    __shared__ int lbase[RS_RADIX];
     __shared__ int sh[32];
     __shared__ long s_tile;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0)
         s_tile = (long)(atomicAdd(ctr, 1ull) - base);
-    for (int i = tid; i < RS_WARPS * RS_RADIX; i += blockDim.x)
+    const int gcount = tid < RS_RADIX ? ghist[tid] : 0;
+    for (int i = tid; i < RS_WARPS * RS_RADIX; i += RS_WARPS * 32)
         (&woff[0][0])[i] = 0;
-    // exclusive scan of the pass's global digit counts
-    int total;
-    const int gex = block_excl_scan(ghist[tid], sh, &total);
     __syncthreads();
     const long tile = s_tile;
     const long wbase = tile * RS_TILE + (long)warp * RS_ITEMS * 32;
+    unsigned k[RS_ITEMS];
+    int v[RS_ITEMS], rank[RS_ITEMS];
+#pragma unroll
     for (int r = 0; r < RS_ITEMS; r++)
     {
         const long i = wbase + r * 32 + lane;
-        if (i < n)
-            atomicAdd(&woff[warp][(kin[i] >> shift) & 0xFF], 1);
+        k[r] = i < n ? kin[i] : 0u;
+        v[r] = i < n ? vin[i] : 0;
+    }
+    // exclusive scan of the pass's global digit counts (the keys are on their way)
+    int total;
+    const int gex = block_excl_scan(gcount, sh, &total);
+    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; r++)
+    {
+        // lanes past the end match each other on a digit that no key has
+        const bool valid = wbase + r * 32 + lane < n;
+        const int dg = valid ? (int)((k[r] >> shift) & 0xFF) : RS_RADIX;
+        const unsigned peers = __match_any_sync(0xffffffffu, dg);
+        const int before = valid ? woff[warp][dg] : 0;
+        rank[r] = before + __popc(peers & lt);
+        __syncwarp();
+        if (valid && (peers & lt) == 0)
+            woff[warp][dg] = before + __popc(peers);
+        __syncwarp();
     }
     __syncthreads();
     // thread d: exclusive prefix over warps of digit d, the tile's count of d
     const int d = tid;
     int cnt = 0;
-    for (int w = 0; w < RS_WARPS; w++)
+    if (d < RS_RADIX)
     {
-        const int c = woff[w][d];
-        woff[w][d] = cnt;
-        cnt += c;
-    }
-    const unsigned long long tag = (unsigned long long)epoch << 32;
-    int prefix = 0;
-    if (tile > 0)
-    {
-        scan_st(&st[tile * RS_RADIX + d], (1ull << 62) | tag | (unsigned)cnt);
-        long polls = 0;
-        for (long j = tile - 1; j >= 0;)
+        for (int w = 0; w < RS_WARPS; w++)
         {
-            const unsigned long long w = scan_ld(&st[j * RS_RADIX + d]);
-            const unsigned fl = (unsigned)(w >> 62);
-            if (fl == 0 || (unsigned)((w >> 32) & 0x3fffffffu) != epoch)
-            {
-                if (++polls > SCAN_POLL_LIMIT)
-                {
-                    atomicOr(&flags[F_ERROR], E_SCAN);
-                    break;
-                }
-                continue;
-            }
-            prefix += (int)(unsigned)w;
-            if (fl == 2)
-                break;
-            j--;
+            const int c = woff[w][d];
+            woff[w][d] = cnt;
+            cnt += c;
         }
+        const unsigned long long tag = (unsigned long long)epoch << 32;
+        scan_st(&st[tile * RS_RADIX + d], ((tile > 0 ? 1ull : 2ull) << 62) | tag | (unsigned)cnt);
     }
-    scan_st(&st[tile * RS_RADIX + d], (2ull << 62) | tag | (unsigned)(prefix + cnt));
-    bbase[d] = gex + prefix;
+    const int lex = block_excl_scan(cnt, sh, &total);
+    if (d < RS_RADIX)
+    {
+        lbase[d] = lex;
+        int prefix = 0;
+        long polls = 0;
+        bool found = tile == 0;
+        for (long j = tile - 1; !found;)
+        {
+            unsigned long long w[RS_BACK];
+#pragma unroll
+            for (int q = 0; q < RS_BACK; q++)
+                w[q] = j - q >= 0 ? scan_ld(&st[(j - q) * RS_RADIX + d]) : 0ull;
+            int used = 0;
+#pragma unroll
+            for (int q = 0; q < RS_BACK; q++)
+            {
+                const unsigned fl = (unsigned)(w[q] >> 62);
+                if (found || used < q || fl == 0 ||
+                    (unsigned)((w[q] >> 32) & 0x3fffffffu) != epoch)
+                    continue;
+                prefix += (int)(unsigned)w[q];
+                found = fl == 2;
+                used++;
+            }
+            j -= used;
+            if (!found && used == 0 && ++polls > SCAN_POLL_LIMIT)
+            {
+                atomicOr(&flags[F_ERROR], E_SCAN);
+                break;
+            }
+        }
+        if (tile > 0)
+            scan_st(&st[tile * RS_RADIX + d],
+                    (2ull << 62) | ((unsigned long long)epoch << 32) | (unsigned)(prefix + cnt));
+        goff[d] = gex + prefix - lex;
+    }
     __syncthreads();
-    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
     for (int r = 0; r < RS_ITEMS; r++)
     {
-        const long i = wbase + r * 32 + lane;
-        const bool valid = i < n;
-        const unsigned active = __ballot_sync(0xffffffffu, valid);
-        if (valid)
+        const int dg = (k[r] >> shift) & 0xFF;
+        rank[r] += lbase[dg] + woff[warp][dg];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; r++)
+        if (wbase + r * 32 + lane < n)
         {
-            const unsigned k = kin[i];
-            const int v = vin[i];
-            const int dg = (k >> shift) & 0xFF;
-            const unsigned peers = __match_any_sync(active, dg);
-            const int rank = __popc(peers & lt);
-            const int pos = bbase[dg] + woff[warp][dg] + rank;
-            kout[pos] = k;
-            vout[pos] = v;
-            __syncwarp(active);
-            if (rank == 0)
-                woff[warp][dg] += __popc(peers);
+            skey[rank[r]] = k[r];
+            sval[rank[r]] = v[r];
         }
-        __syncwarp();
+    __syncthreads();
+    const int here = (int)(n - tile * RS_TILE < RS_TILE ? n - tile * RS_TILE : RS_TILE);
+#pragma unroll
+    for (int r = 0; r < RS_ITEMS; r++)
+    {
+        const int at = tid + r * RS_WARPS * 32;
+        if (at < here)
+        {
+            const unsigned key = skey[at];
+            const int pos = goff[(key >> shift) & 0xFF] + at;
+            kout[pos] = key;
+            vout[pos] = sval[at];
+        }
     }
 }
 
@@ -365,6 +415,86 @@ int scan_exclusive(qz_sim *s, const int *in, int *out, long n)
            n, s->scan_st, s->scan_st + s->scan_st_cap, s->scan_base, s->scan_epoch, s->flags);
     s->scan_base += (unsigned long long)tiles;
     return check_cuda(cudaGetLastError(), "scan") ? QZ_SUCCESS : QZ_FAILURE;
+}
+
+// Cell segments of n sorted keys in one launch: a single-pass scan (as
+// k_scan_lookback) of the flags "differs from the key before", each head writing its
+// segment's first position and key and the cell's segment; the last element closes the
+// table, writes flags[F_NSEG] and clears flags[F_NLONG].
+__global__ void __launch_bounds__(SC_THREADS)
+    k_seg_build(const unsigned *__restrict__ k, long n, unsigned morton_B,
+                int *__restrict__ seg_start, int *__restrict__ seg_cell, int *__restrict__ cell_seg,
+                unsigned long long *__restrict__ st, unsigned long long *__restrict__ ctr,
+                unsigned long long base, unsigned epoch, int *__restrict__ flags)
+{
+    __shared__ int sh[32];
+    __shared__ long s_tile;
+    __shared__ int s_prefix;
+    if (threadIdx.x == 0)
+        s_tile = (long)(atomicAdd(ctr, 1ull) - base);
+    __syncthreads();
+    const long tile = s_tile;
+    const long i0 = tile * SC_TILE + (long)threadIdx.x * SC_ITEMS;
+    unsigned key[SC_ITEMS + 1]; // from the key before
+    key[0] = i0 > 0 && i0 <= n ? k[i0 - 1] : 0u;
+    bool head[SC_ITEMS];
+    int sum = 0;
+    for (int q = 0; q < SC_ITEMS; q++)
+    {
+        const long i = i0 + q;
+        key[q + 1] = i < n ? k[i] : 0u;
+        head[q] = i < n && (i == 0 || key[q + 1] != key[q]);
+        sum += head[q];
+    }
+    int total;
+    const int ex = block_excl_scan(sum, sh, &total);
+    if (threadIdx.x < 32)
+    {
+        const unsigned long long tag = (unsigned long long)epoch << 32;
+        int prefix = 0;
+        if (tile > 0)
+        {
+            if (threadIdx.x == 0)
+                scan_st(&st[tile], (1ull << 62) | tag | (unsigned)total);
+            prefix = scan_lookback_warp(st, tile, epoch, flags);
+        }
+        if (threadIdx.x == 0)
+        {
+            scan_st(&st[tile], (2ull << 62) | tag | (unsigned)(prefix + total));
+            s_prefix = prefix;
+        }
+    }
+    __syncthreads();
+    int sg = s_prefix + ex;
+    for (int q = 0; q < SC_ITEMS; q++)
+    {
+        const long i = i0 + q;
+        if (head[q])
+        {
+            seg_start[sg] = (int)i;
+            seg_cell[sg] = (int)key[q + 1];
+            cell_seg[key_cell(key[q + 1], morton_B)] = sg;
+            sg++;
+        }
+        if (i == n - 1)
+        {
+            seg_start[sg] = (int)n;
+            flags[F_NSEG] = sg;
+            flags[F_NLONG] = 0;
+        }
+    }
+}
+
+int seg_build(qz_sim *s, const unsigned *keys, long n, unsigned morton_B, int *cell_seg)
+{
+    const long tiles = (n + SC_TILE - 1) / SC_TILE;
+    if (scan_prepare(s, tiles))
+        return QZ_FAILURE;
+    launch(s, QZ_PROF_DEPOSIT, 12.0 * n, k_seg_build, dim3((int)tiles), dim3(SC_THREADS), keys, n,
+           morton_B, s->seg_start, s->seg_cell, cell_seg, s->scan_st, s->scan_st + s->scan_st_cap,
+           s->scan_base, s->scan_epoch, s->flags);
+    s->scan_base += (unsigned long long)tiles;
+    return check_cuda(cudaGetLastError(), "cell segments") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
 // Sorts s->sort.k0/v0 (n pairs) on the low `bits` bits; the sorted result is
