@@ -3160,7 +3160,8 @@ int amr_grid_accel(qz_sim *s)
 __global__ void k_amr_gather(long n, LevelRefs R, const double *__restrict__ x,
                              const double *__restrict__ y, const double *__restrict__ z,
                              double *__restrict__ pax, double *__restrict__ pay,
-                             double *__restrict__ paz, int *__restrict__ flags)
+                             double *__restrict__ paz, int *__restrict__ flags, bool fresh,
+                             Kick kick)
 {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -3183,6 +3184,8 @@ __global__ void k_amr_gather(long n, LevelRefs R, const double *__restrict__ x,
     if (!(px >= 0.0 && py >= 0.0 && pz >= 0.0) || b < 0 || b >= (long)N.rd[0] * N.rd[1] * N.rd[2])
     {
         atomicOr(&flags[F_ERROR], E_PTCL_OUTSIDE);
+        if (fresh)
+            pax[i] = pay[i] = paz[i] = 0.0;
         return;
     }
     double wx1 = px - fx, wy1 = py - fy, wz1 = pz - fz;
@@ -3199,7 +3202,7 @@ __global__ void k_amr_gather(long n, LevelRefs R, const double *__restrict__ x,
     const long sx = N.rd[0] + 1, sxy = sx * (N.rd[1] + 1);
     const long g = grid_index(N, fx - N.ts[0], fy - N.ts[1], fz - N.ts[2]);
     const double *gx = R.ax[l], *gy = R.ay[l], *gz = R.az[l];
-    double ax = pax[i], ay = pay[i], az = paz[i];
+    double ax = fresh ? 0.0 : pax[i], ay = fresh ? 0.0 : pay[i], az = fresh ? 0.0 : paz[i];
 #pragma unroll
     for (int kk = 0; kk < 2; kk++)
 #pragma unroll
@@ -3216,6 +3219,7 @@ __global__ void k_amr_gather(long n, LevelRefs R, const double *__restrict__ x,
     pax[i] = ax;
     pay[i] = ay;
     paz[i] = az;
+    apply_kick(kick, i, ax, ay, az);
 }
 
 // observables.c:205-424: m times the potential interpolated (CIC) at the
@@ -3284,7 +3288,7 @@ int amr_pot_energy_partials(qz_sim *s, double *part)
     return check_cuda(cudaGetLastError(), "potential energy") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
-int amr_gather(qz_sim *s)
+int amr_gather(qz_sim *s, bool fresh, double kick_dt)
 {
     if (s->n == 0)
         return QZ_SUCCESS;
@@ -3300,7 +3304,7 @@ int amr_gather(qz_sim *s)
     }
     launch(s, QZ_PROF_GATHER, 72.0 * s->n + 8.0 * s->n * s->amr_nlev, k_amr_gather,
            dim3(blocks_for(s->n, 256)), dim3(256), s->n, R, s->x, s->y, s->z, s->ax, s->ay, s->az,
-           s->flags);
+           s->flags, fresh, Kick{kick_dt, s->vx, s->vy, s->vz});
     return check_cuda(cudaGetLastError(), "amr gather") ? QZ_SUCCESS : QZ_FAILURE;
 }
 } // namespace qz

@@ -125,10 +125,9 @@ static bool build_levels(qz_sim *s, int n0)
     const bool cgs = s->cfg.smoother == 2;
     if (cgs && !s->cg_part && !dmalloc(&s->cg_part, 2 * QZ_CG_PART_MAX, "cg partials"))
         return false;
-    // persistent cycles: per-block partials of the in-launch convergence test, its result
-    if (!s->mg_part && !dmalloc(&s->mg_part, 2 * QZ_CG_PART_MAX + 8, "mg partials"))
+    // persistent cycles: per-block partials of the in-launch convergence test
+    if (!s->mg_part && !dmalloc(&s->mg_part, 2 * QZ_CG_PART_MAX, "mg partials"))
         return false;
-    cudaMemset(s->mg_part, 0, (2 * QZ_CG_PART_MAX + 8) * sizeof(double));
     for (auto &l : s->levels)
     {
         size_t pts = (size_t)l.n * l.n * l.n;
@@ -534,8 +533,9 @@ int qz_create(const qz_config *cfg, long n_capacity, qz_sim **out)
          dmalloc(&s->cell_seg, B * B * B, "cell_seg") && dmalloc(&s->cell_sums, 8 * cap, "cs") &&
          dmalloc(&s->long_seg, cap / SEG_LONG + 2, "long segments");
     s->red_blocks = 296;
-    ok = ok && dmalloc(&s->red, s->red_blocks + 8, "red") && dmalloc(&s->flags, F_COUNT, "flags");
-    ok = ok && check_cuda(cudaMallocHost((void **)&s->h_flags, F_COUNT * sizeof(int)), "pinned");
+    ok = ok && dmalloc(&s->red, s->red_blocks + 8, "red") && dmalloc(&s->flags, F_COUNT + F_OUTST, "flags");
+    s->outst = s->flags + F_COUNT;
+    ok = ok && check_cuda(cudaMallocHost((void **)&s->h_flags, (F_COUNT + F_OUTST) * sizeof(int)), "pinned");
     ok = ok && dmalloc(&s->gbar, 4, "grid barrier");
     ok = ok && check_cuda(cudaMallocHost((void **)&s->h_ts, 34 * sizeof(unsigned long long)),
                           "pinned time step") &&
@@ -544,7 +544,7 @@ int qz_create(const qz_config *cfg, long n_capacity, qz_sim **out)
     s->sort.tiles_cap = tiles;
     if (ok)
     {
-        cudaMemset(s->flags, 0, F_COUNT * sizeof(int));
+        cudaMemset(s->flags, 0, (F_COUNT + F_OUTST) * sizeof(int));
         size_t gb = s->gpts * sizeof(double);
         cudaMemset(s->pot_old, 0, gb);
         cudaMemset(s->d, 0, gb);
@@ -873,13 +873,20 @@ static int tree_density_potential(qz_sim *s, StepPending &sp)
     return amr_potential(s);
 }
 
+// The gather and the kick of a step in one launch, from zero accelerations; with it a step
+// needs no reset (reset.c:29-64): the deposit writes every point of the head's density.
+static int gather_kick(qz_sim *s, double dt)
+{
+    return amr_on(s) ? amr_gather(s, true, dt) : gather_head(s, true, dt);
+}
+
 // main.c:375-481 with a given dt: kick-drift, reset, tree, deposit, potential,
 // gradient, gather, kick.
 int step_core(qz_sim *s, double h)
 {
     StepPending sp;
-    const bool ok = !kick_drift(s, h) && !qz_reset(s) && !tree_density_potential(s, sp) &&
-                    !qz_grid_acceleration(s) && !qz_particle_acceleration(s) && !kick(s, h);
+    const bool ok = !kick_drift(s, h) && !tree_density_potential(s, sp) &&
+                    !qz_grid_acceleration(s) && !gather_kick(s, h);
     if (step_finish(s, sp) || !ok)
         return QZ_FAILURE;
     s->stats.steps++;
@@ -1003,10 +1010,9 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
         if (!check_cuda(cudaMemcpyAsync(hx[q], dx[q], b, cudaMemcpyDeviceToHost, s->xfer), "d2h"))
             return QZ_FAILURE;
     StepPending sp;
-    const bool ok = !qz_reset(s) &&
-                    check_cuda(cudaStreamWaitEvent(s->stream, s->ev_mass, 0), "wait") &&
+    const bool ok = check_cuda(cudaStreamWaitEvent(s->stream, s->ev_mass, 0), "wait") &&
                     !tree_density_potential(s, sp) && !qz_grid_acceleration(s) &&
-                    !qz_particle_acceleration(s) && !kick(s, dt);
+                    !gather_kick(s, dt);
     // the copies back are queued before the step's outcomes are read
     double *ho[6] = {vx, vy, vz, ax, ay, az};
     const double *dout[6] = {s->vx, s->vy, s->vz, s->ax, s->ay, s->az};

@@ -179,12 +179,14 @@ template <int LG> struct DirectShape {
     static constexpr int T = N / 4;                               // threads of a pair
     static constexpr int THREADS = P * T;
     static constexpr size_t SMEM = sizeof(Cplx) * P * (2 * N + N / 4);
+    // 64 registers a thread: the passes wait for their loads, so warps count
+    static constexpr int BLOCKS = 1024 / THREADS < 1 ? 1 : 1024 / THREADS > 16 ? 16 : 1024 / THREADS;
 };
 
 // x passes: pairs of rows (j = 2 p, 2 p + 1) of plane k.  FORWARD: r of phi into w, else
 // phi += the transform of w.
 template <int LG, bool FORWARD>
-__global__ void __launch_bounds__(DirectShape<LG>::THREADS)
+__global__ void __launch_bounds__(DirectShape<LG>::THREADS, DirectShape<LG>::BLOCKS)
     k_sine_x(Grid<double> phi, Grid<double> rho, double *__restrict__ w,
              const double2 *__restrict__ tw, const int *__restrict__ done)
 {
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(DirectShape<LG>::THREADS)
 // y passes (stride N, plane blockIdx.y) and the z pass (stride N^2, row blockIdx.y): pairs of
 // adjacent x.  The z pass divides by the eigenvalues between its two transforms.
 template <int LG, bool SOLVE>
-__global__ void __launch_bounds__(DirectShape<LG>::THREADS)
+__global__ void __launch_bounds__(DirectShape<LG>::THREADS, DirectShape<LG>::BLOCKS)
     k_sine_yz(double *__restrict__ w, const double2 *__restrict__ tw,
               const double *__restrict__ lam, const int *__restrict__ done)
 {
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(DirectShape<LG>::THREADS)
 constexpr int DC_THREADS = 256;
 
 __global__ void __launch_bounds__(DC_THREADS)
-    k_direct_check(int nc, int D, const double *__restrict__ pot, double *__restrict__ pot_old,
+    k_direct_check(int nc, unsigned D, unsigned inv, const double *__restrict__ pot, double *__restrict__ pot_old,
                    const double *__restrict__ d, double rm, double tol, int method, double nintr,
                    double *__restrict__ part, int *__restrict__ outst, bool again)
 {
@@ -302,13 +304,13 @@ __global__ void __launch_bounds__(DC_THREADS)
         return;
     __shared__ double sh[DC_THREADS / 32];
     __shared__ int sh_last;
-    const unsigned total = (unsigned)D * D * D, D2 = (unsigned)D * D;
+    const unsigned D2 = D * D, k = blockIdx.y;
     const double oh2 = (double)nc * nc;
     double acc = 0.0;
     int fail = 0;
-    for (unsigned g = blockIdx.x * DC_THREADS + threadIdx.x; g < total; g += gridDim.x * DC_THREADS)
+    for (unsigned q = blockIdx.x * DC_THREADS + threadIdx.x; q < D2; q += gridDim.x * DC_THREADS)
     {
-        const unsigned k = g / D2, rest = g - k * D2, j = rest / D, i = rest - j * D;
+        const unsigned j = __umulhi(q, inv), i = q - j * D, g = k * D2 + q;
         const double c = pot[g];
         pot_old[g] = c;
         if (i < 2 || j < 2 || k < 2 || i > (unsigned)nc || j > (unsigned)nc || k > (unsigned)nc)
@@ -337,16 +339,16 @@ __global__ void __launch_bounds__(DC_THREADS)
     acc = block_sum(acc);
     if (threadIdx.x == 0)
     {
-        part[blockIdx.x] = acc;
+        part[blockIdx.y * gridDim.x + blockIdx.x] = acc;
         __threadfence();
-        sh_last = atomicAdd(&outst[3], 1) == (int)gridDim.x - 1;
+        sh_last = atomicAdd(&outst[3], 1) == (int)(gridDim.x * gridDim.y) - 1;
     }
     __syncthreads();
     if (!sh_last)
         return;
     __threadfence();
     double t = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += DC_THREADS)
+    for (int b = threadIdx.x; b < (int)(gridDim.x * gridDim.y); b += DC_THREADS)
         t += __ldcg(part + b);
     t = block_sum(t);
     if (threadIdx.x == 0)
@@ -459,11 +461,13 @@ static int direct_check(qz_sim *s, bool again)
     const double H = 1.0 / nc;
     const double rm = 4.0 * c.G * 3.14159265358979323846 * s->head_mass / ((double)nc * nc * nc * H * H * H);
     const double m = nc - 1;
-    int *outst = reinterpret_cast<int *>(s->mg_part + 2 * QZ_CG_PART_MAX);
-    const int blocks = (int)std::min<long>(QZ_CG_PART_MAX, blocks_for(s->gpts, 4 * DC_THREADS));
-    launch(s, QZ_PROF_CHECK, 24.0 * s->gpts, k_direct_check, dim3(blocks), dim3(DC_THREADS), nc,
-           (int)s->D, s->pot, s->pot_old, s->d, rm, c.tol, c.check_method, m * m * m, s->mg_part,
-           outst, again);
+    const unsigned D = (unsigned)s->D;
+    // a plane of points a row of blocks; the partials' buffer holds 2 x QZ_CG_PART_MAX
+    const unsigned bx = std::max(1u, std::min((D * D + 4 * DC_THREADS - 1) / (4 * DC_THREADS),
+                                              2 * QZ_CG_PART_MAX / D));
+    launch(s, QZ_PROF_CHECK, 24.0 * s->gpts, k_direct_check, dim3(bx, D), dim3(DC_THREADS), nc, D,
+           div_magic(D), s->pot, s->pot_old, s->d, rm, c.tol, c.check_method, m * m * m, s->mg_part,
+           s->outst, again);
     return check_cuda(cudaGetLastError(), "direct solve test") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
@@ -473,7 +477,7 @@ static int direct_check(qz_sim *s, bool again)
 // that grows with N^2, of the order of the default tolerance there.
 int direct_head(qz_sim *s)
 {
-    const int *done = reinterpret_cast<const int *>(s->mg_part + 2 * QZ_CG_PART_MAX) + 2;
+    const int *done = s->outst + 2;
     if (direct_correct(s, s->pot, s->d) || direct_check(s, false))
         return QZ_FAILURE;
     return s->L >= 8 && (direct_correct_unless(s, s->pot, s->d, done) || direct_check(s, true))

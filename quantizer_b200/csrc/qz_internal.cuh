@@ -121,6 +121,23 @@ __device__ __forceinline__ long key_cell(unsigned k, unsigned morton_B)
 
 #endif
 
+// The kick of half a step (particle_updating.c:2677-2688) that a gather applies to its
+// particle when dt is not zero.
+struct Kick {
+    double dt;
+    double *vx, *vy, *vz;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void apply_kick(const Kick &k, long i, double ax, double ay, double az)
+{
+    if (k.dt == 0.0)
+        return;
+    k.vx[i] += ax * k.dt * 0.5;
+    k.vy[i] += ay * k.dt * 0.5;
+    k.vz[i] += az * k.dt * 0.5;
+}
+#endif
+
 // Device-side flag words (int).
 enum Flag {
     F_RATIO_FAIL = 0, // ratio test |phi/phi_old - 1| > tol2 somewhere
@@ -130,7 +147,8 @@ enum Flag {
     F_RESID_FAIL = 4, // method-1 pointwise residual failure
     F_AMR_CONV = 5,   // refinement nodes converged in the current level solve
     F_NLONG = 6,      // deposit segments longer than SEG_LONG (listed in long_seg)
-    F_COUNT = 8
+    F_COUNT = 8,
+    F_OUTST = 4 // words of outst, after the flags
 };
 enum ErrorBits { E_PTCL_OUTSIDE = 1, E_SORT_RANGE = 2, E_BARRIER = 8, E_SCAN = 16 };
 
@@ -185,8 +203,25 @@ __device__ __forceinline__ void seg_sums(int nseg, const int *__restrict__ perm,
         for (int c = 0; c < NV; c++)
             acc[c] = 0.0;
         const int gl = lane & (W - 1);
-        for (int q = b + gl; q < e; q += W)
-            add(perm[q], acc);
+        if constexpr (W < 32)
+        {
+            if (b + gl < e)
+                add(perm[b + gl], acc);
+        }
+        else
+        {
+            for (int q0 = b + gl; q0 < e; q0 += 4 * W) // four particles' loads together
+            {
+                int id[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    id[u] = q0 + u * W < e ? perm[q0 + u * W] : -1;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (id[u] >= 0)
+                        add(id[u], acc);
+            }
+        }
 #pragma unroll
         for (int k = 0; k < NC; k++)
         {
@@ -203,6 +238,21 @@ __device__ __forceinline__ void seg_sums(int nseg, const int *__restrict__ perm,
                 put(sg, NV - 1, v);
         }
     };
+    auto whole = [&](long sg, int b, int e) {
+        if (e - b > SEG_LONG)
+        {
+            if (lane == 0)
+                long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sg;
+        }
+        else
+            group(std::integral_constant<int, 32>{}, sg, b, e);
+    };
+    if (nseg <= nwarps) // warps for all cells: grouping would only make some wait
+    {
+        for (long sg = warp0; sg < nseg; sg += nwarps)
+            whole(sg, seg_start[sg], seg_start[sg + 1]);
+        return;
+    }
     for (long s4 = warp0 * 4; s4 < nseg; s4 += nwarps * 4)
     {
         const long sg = s4 + (lane >> 3);
@@ -232,13 +282,7 @@ __device__ __forceinline__ void seg_sums(int nseg, const int *__restrict__ perm,
                 const long sw = s4 + 2 * h + u;
                 const int bw = __shfl_sync(0xffffffffu, bp, 16 * u),
                           ew = __shfl_sync(0xffffffffu, ep, 16 * u);
-                if (ew - bw > SEG_LONG)
-                {
-                    if (lane == 0)
-                        long_list[atomicAdd(&flags[F_NLONG], 1)] = (int)sw;
-                    continue;
-                }
-                group(std::integral_constant<int, 32>{}, sw, bw, ew);
+                whole(sw, bw, ew);
             }
         }
     }
@@ -528,8 +572,9 @@ struct qz_sim {
 
     double *red = nullptr; // reduction partials
     int red_blocks = 0;
-    int *flags = nullptr;  // device flag words
-    int *h_flags = nullptr; // pinned mirror
+    int *flags = nullptr;  // device flag words, then the head solve's outcome (outst)
+    int *outst = nullptr;  // head solve: cycles run, converged, direct solve passed, counter
+    int *h_flags = nullptr; // pinned mirror of both
     unsigned long long *d_ts = nullptr; // time-step reduction words (17)
     unsigned long long *h_ts = nullptr; // pinned: 17 words out, 17 back
     double *h_red = nullptr; // pinned scalar readback
@@ -696,7 +741,9 @@ int grid_accel_head_from(qz_sim *s, const double *pot);
 int head_segments(qz_sim *s, const double *x, const double *y, const double *z, int **perm_out);
 int deposit_segments(qz_sim *s, long m, int bits, int *cell_seg, long ncells_box,
                      unsigned **ks_out, int **perm_out, unsigned morton_B);
-int gather_head(qz_sim *s);
+// fresh: the accelerations start from zero instead of adding to the arrays; kick_dt != 0:
+// the kick of half a step follows in the same launch
+int gather_head(qz_sim *s, bool fresh = false, double kick_dt = 0.0);
 int kick_drift(qz_sim *s, double dt);
 int kick(qz_sim *s, double dt);
 
@@ -725,7 +772,7 @@ bool amr_potential_queues(const qz_sim *s);
 int amr_potential_issue(qz_sim *s, std::vector<CgPending> &pend);
 int amr_potential_collect(qz_sim *s, const std::vector<CgPending> &pend);
 int amr_grid_accel(qz_sim *s);
-int amr_gather(qz_sim *s);
+int amr_gather(qz_sim *s, bool fresh = false, double kick_dt = 0.0);
 int poisson_error_head(qz_sim *s, int *converged);
 bool head_one_launch(const qz_sim *s);
 int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued);
@@ -765,6 +812,10 @@ inline Grid<T> dense_view(T *p, int n)
     g.n = n;
     return g;
 }
+
+// q / d = __umulhi(q, div_magic(d)) for q < 2^32 / d (the error of the rounded-up
+// reciprocal stays below 1 / d): points of a plane of a head grid, d its side.
+inline unsigned div_magic(unsigned d) { return (unsigned)((0x100000000ULL + d - 1) / d); }
 
 inline int blocks_for(long n, int threads)
 {

@@ -309,38 +309,28 @@ __global__ void __launch_bounds__(SEG_LONG_THREADS)
 
 // Each grid point sums the corner contributions of its (up to) 8 adjacent
 // occupied cells in a fixed order.
-__global__ void k_point_gather(int L, long D, const int *__restrict__ cell_seg,
+// blockIdx.y is the plane; the eight cells' segments are loaded together.
+__global__ void k_point_gather(int D, unsigned inv, const int *__restrict__ cell_seg,
                                const double *__restrict__ cs, double *__restrict__ d)
 {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, uD = (unsigned)D;
-    if (t >= uD * uD * uD)
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (unsigned)(D * D))
         return;
-    const long B = D - 1;
-    const unsigned q = t / uD, r = q / uD;
-    const int gx = (int)(t - q * uD), gy = (int)(q - r * uD), gz = (int)r;
-    double acc = 0.0;
-    for (int c = 0; c < 2; c++)
+    const int B = D - 1, gz = (int)blockIdx.y, gy = (int)__umulhi(q, inv), gx = (int)q - gy * D;
+    int sg[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++)
     {
-        int cz = gz - 1 + c;
-        if (cz < 0 || cz >= B)
-            continue;
-        for (int b = 0; b < 2; b++)
-        {
-            int cy = gy - 1 + b;
-            if (cy < 0 || cy >= B)
-                continue;
-            for (int a = 0; a < 2; a++)
-            {
-                int cx = gx - 1 + a;
-                if (cx < 0 || cx >= B)
-                    continue;
-                int sg = cell_seg[cx + cy * B + (long)cz * B * B];
-                if (sg >= 0)
-                    acc += cs[(long)sg * 8 + (1 - a) + 2 * (1 - b) + 4 * (1 - c)];
-            }
-        }
+        const int cx = gx - 1 + (o & 1), cy = gy - 1 + ((o >> 1) & 1), cz = gz - 1 + (o >> 2);
+        const bool in = cx >= 0 && cx < B && cy >= 0 && cy < B && cz >= 0 && cz < B;
+        sg[o] = in ? cell_seg[cx + (cy + cz * B) * B] : -1;
     }
-    d[t] = acc;
+    double acc = 0.0;
+#pragma unroll
+    for (int o = 0; o < 8; o++)
+        if (sg[o] >= 0)
+            acc += cs[(long)sg[o] * 8 + (7 - o)];
+    d[(unsigned)gz * (unsigned)(D * D) + q] = acc;
 }
 
 // Sorts the m (cell key, particle) pairs staged in s->sort.k0 / v0 and builds
@@ -418,7 +408,9 @@ int deposit_head(qz_sim *s)
            s->seg_start, s->flags, s->long_seg, s->x, s->y, s->z, s->m, s->cell_sums);
     launch(s, QZ_PROF_DEPOSIT, 0.0, k_seg_long, dim3(sms), dim3(SEG_LONG_THREADS), L, coeff, perm,
            s->seg_start, s->flags, s->long_seg, s->x, s->y, s->z, s->m, s->cell_sums);
-    launch(s, QZ_PROF_DEPOSIT, 12.0 * s->gpts, k_point_gather, dim3(blocks_for(s->gpts, 256)), dim3(256), L, s->D, s->cell_seg, s->cell_sums, s->d);
+    launch(s, QZ_PROF_DEPOSIT, 12.0 * s->gpts, k_point_gather,
+           dim3(blocks_for(s->D * s->D, 256), (unsigned)s->D), dim3(256), (int)s->D,
+           div_magic((unsigned)s->D), s->cell_seg, s->cell_sums, s->d);
     return check_cuda(cudaGetLastError(), "deposit") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
@@ -502,7 +494,7 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
                               const double *__restrict__ gx, const double *__restrict__ gy,
                               const double *__restrict__ gz, double *__restrict__ pax,
                               double *__restrict__ pay, double *__restrict__ paz,
-                              int *__restrict__ flags)
+                              int *__restrict__ flags, bool fresh, Kick kick)
 {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -514,6 +506,8 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
         fz > (1 << L))
     {
         atomicOr(&flags[F_ERROR], E_PTCL_OUTSIDE);
+        if (fresh)
+            pax[i] = pay[i] = paz[i] = 0.0;
         return;
     }
     double wx1 = px - fx, wy1 = py - fy, wz1 = pz - fz;
@@ -529,7 +523,7 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
     w[7] = wx1 * wy1 * wz1;
     const long D2 = D * D;
     long g = (fx + 1) + (long)(fy + 1) * D + (long)(fz + 1) * D2;
-    double ax = pax[i], ay = pay[i], az = paz[i];
+    double ax = fresh ? 0.0 : pax[i], ay = fresh ? 0.0 : pay[i], az = fresh ? 0.0 : paz[i];
 #pragma unroll
     for (int kk = 0; kk < 2; kk++)
 #pragma unroll
@@ -546,13 +540,14 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
     pax[i] = ax;
     pay[i] = ay;
     paz[i] = az;
+    apply_kick(kick, i, ax, ay, az);
 }
 
-int gather_head(qz_sim *s)
+int gather_head(qz_sim *s, bool fresh, double kick_dt)
 {
     if (s->n == 0)
         return QZ_SUCCESS;
-    launch(s, QZ_PROF_GATHER, 72.0 * s->n + 24.0 * s->gpts, k_gather_head, dim3(blocks_for(s->n, 256)), dim3(256), s->n, s->L, s->D, s->x, s->y, s->z, s->gax, s->gay, s->gaz, s->ax, s->ay, s->az, s->flags);
+    launch(s, QZ_PROF_GATHER, 72.0 * s->n + 24.0 * s->gpts, k_gather_head, dim3(blocks_for(s->n, 256)), dim3(256), s->n, s->L, s->D, s->x, s->y, s->z, s->gax, s->gay, s->gaz, s->ax, s->ay, s->az, s->flags, fresh, Kick{kick_dt, s->vx, s->vy, s->vz});
     return check_cuda(cudaGetLastError(), "gather") ? QZ_SUCCESS : QZ_FAILURE;
 }
 

@@ -1897,7 +1897,7 @@ static int mg_launch(qz_sim *s, int iters, bool check = false, bool defer = fals
         const double H = 1.0 / nc;
         A.pold = s->pot_old;
         A.part = s->mg_part;
-        A.outst = reinterpret_cast<int *>(s->mg_part + 2 * QZ_CG_PART_MAX);
+        A.outst = s->outst;
         A.tm = 1.0 - c.tol2;
         A.tp = 1.0 + c.tol2;
         A.rm = 4.0 * c.G * QZ_PI_D * s->head_mass / ((double)nc * nc * nc * H * H * H);
@@ -2524,11 +2524,8 @@ int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued)
 // the test's outcome and the barrier status.
 int potential_head_finish(qz_sim *s, cudaStream_t st)
 {
-    int out[2] = {0, 0};
-    const int *outst = reinterpret_cast<const int *>(s->mg_part + 2 * QZ_CG_PART_MAX);
-    if (!check_cuda(cudaMemcpyAsync(out, outst, sizeof out, cudaMemcpyDeviceToHost, st),
-                    "multigrid result") ||
-        !check_cuda(cudaMemcpyAsync(s->h_flags, s->flags, F_COUNT * sizeof(int),
+    const int *out = s->h_flags + F_COUNT;
+    if (!check_cuda(cudaMemcpyAsync(s->h_flags, s->flags, (F_COUNT + F_OUTST) * sizeof(int),
                                     cudaMemcpyDeviceToHost, st),
                     "flags") ||
         !check_cuda(cudaStreamSynchronize(st), "multigrid result"))
@@ -2561,9 +2558,8 @@ int potential_head(qz_sim *s)
     if (head_direct(s))
     {
         int ok = 0;
-        const int *outst = reinterpret_cast<const int *>(s->mg_part + 2 * QZ_CG_PART_MAX);
         if (direct_head(s) ||
-            !check_cuda(cudaMemcpyAsync(&ok, outst + 2, sizeof ok, cudaMemcpyDeviceToHost,
+            !check_cuda(cudaMemcpyAsync(&ok, s->outst + 2, sizeof ok, cudaMemcpyDeviceToHost,
                                         s->stream), "direct solve result") ||
             !check_cuda(cudaStreamSynchronize(s->stream), "direct solve result"))
             return QZ_FAILURE;
