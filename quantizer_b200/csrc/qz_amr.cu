@@ -71,34 +71,113 @@ __device__ __forceinline__ double block_sum_d(double v, double *sh)
     return r;
 }
 
-// ---- tree: counts, flags, zones ------------------------------------------------------
-__global__ void k_fill_int(long n, int *a, int v)
+// ---- ordered selection ------------------------------------------------------------------
+// Items selected from a list keep their order.  The selecting kernel leaves one count a
+// block of SEL_THREADS items, the counts are scanned, and the kernel that uses the items
+// finds an item's place as its block's scanned count plus its rank in the block.  A flag
+// and a place an item (12 bytes written and read, and a scan of as many items: 60 us for
+// the 9.2 million points' flags of a level of a 256^3 run) become 1/256 of that.
+constexpr int SEL_THREADS = 256;
+constexpr int SEL_WARPS = SEL_THREADS / 32;
+
+// Number of the block's threads with `on` set (every thread calls; *rank: those before
+// this one).  sh: SEL_WARPS words that no other call of the kernel uses.
+__device__ __forceinline__ int sel_rank(bool on, int *sh, int *rank)
 {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        a[i] = v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (lane == 0)
+        sh[warp] = __popc(m);
+    __syncthreads();
+    int before = __popc(m & ((1u << lane) - 1u)), total = 0;
+#pragma unroll
+    for (int w = 0; w < SEL_WARPS; w++)
+    {
+        before += w < warp ? sh[w] : 0;
+        total += sh[w];
+    }
+    *rank = before;
+    return total;
 }
 
-__global__ void k_count(long n, const int *__restrict__ node_of, const AmrNode *__restrict__ nodes,
-                        const double *__restrict__ x, const double *__restrict__ y,
-                        const double *__restrict__ z, int *__restrict__ cnt, int *__restrict__ flags)
+constexpr int READ_FEW = 32;
+struct ReadList {
+    const int *at[READ_FEW];
+};
+
+// A few device ints to pinned host memory.
+__global__ void k_read_few(int m, ReadList L, int *__restrict__ out)
 {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
+    const int q = threadIdx.x;
+    if (q < m)
+        out[q] = *L.at[q];
+}
+
+// ---- tree: counts, flags, zones ------------------------------------------------------
+// Statuses of the head's box (initialization.c:95-110): -5 on the ghost ring, -3 inside;
+// and the particle counts' start.
+__global__ void k_head_box(int B, int *__restrict__ box, int *__restrict__ cnt)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (p >= B * B)
         return;
-    int nd = node_of[i];
-    if (nd < 0)
-        return;
-    const AmrNode N = nodes[nd];
-    const double sc = (double)(1 << N.lv);
-    int cx = (int)(x[i] * sc), cy = (int)(y[i] * sc), cz = (int)(z[i] * sc);
-    long b = box_index(N, cx, cy, cz);
-    if (b < 0 || b >= (long)N.rd[0] * N.rd[1] * N.rd[2])
+    const int j = p / B, i = p - j * B;
+    const bool in = i > 0 && i < B - 1 && j > 0 && j < B - 1 && k > 0 && k < B - 1;
+    const long b = p + (long)B * B * k;
+    box[b] = in ? -3 : -5;
+    cnt[b] = 0;
+}
+
+// Particles per cell.  A block adds up COUNT_ITEMS particles a thread in a table of cells
+// in shared memory (a cell whose place in the table is another's goes to memory at once):
+// the densest cells, whose additions in memory run one after the other, are added to once
+// a block.  A million particles, 1.4% of them in each of the eight densest cells: 22 us,
+// 53 with an addition in memory each; below about 300,000 the two take the same.
+constexpr int COUNT_THREADS = 256, COUNT_ITEMS = 8, COUNT_PLACES = 1024;
+
+__global__ void __launch_bounds__(COUNT_THREADS)
+    k_count(long n, const int *__restrict__ node_of, const AmrNode *__restrict__ nodes,
+            const double *__restrict__ x, const double *__restrict__ y,
+            const double *__restrict__ z, int *__restrict__ cnt, int *__restrict__ flags)
+{
+    __shared__ long cell[COUNT_PLACES];
+    __shared__ int sum[COUNT_PLACES];
+    for (int q = threadIdx.x; q < COUNT_PLACES; q += COUNT_THREADS)
     {
-        atomicOr(&flags[F_ERROR], E_PTCL_OUTSIDE);
-        return;
+        cell[q] = -1;
+        sum[q] = 0;
     }
-    atomicAdd(&cnt[N.box_off + b], 1);
+    __syncthreads();
+    const long i0 = (long)blockIdx.x * (COUNT_THREADS * COUNT_ITEMS) + threadIdx.x;
+#pragma unroll 4
+    for (int q = 0; q < COUNT_ITEMS; q++)
+    {
+        const long i = i0 + q * COUNT_THREADS;
+        const int nd = i < n ? node_of[i] : -1;
+        if (nd < 0)
+            continue;
+        const AmrNode &N = nodes[nd];
+        const double sc = (double)(1 << N.lv);
+        const int cx = (int)(x[i] * sc), cy = (int)(y[i] * sc), cz = (int)(z[i] * sc);
+        const long b = box_index(N, cx, cy, cz);
+        if (b < 0 || b >= (long)N.rd[0] * N.rd[1] * N.rd[2])
+        {
+            atomicOr(&flags[F_ERROR], E_PTCL_OUTSIDE);
+            continue;
+        }
+        const long at = N.box_off + b;
+        const int place = (int)(((unsigned)at * 2654435761u) >> 22);
+        const long was = (long)atomicCAS((unsigned long long *)&cell[place],
+                                         (unsigned long long)-1L, (unsigned long long)at);
+        if (was == -1 || was == at)
+            atomicAdd(&sum[place], 1);
+        else
+            atomicAdd(&cnt[at], 1);
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < COUNT_PLACES; q += COUNT_THREADS)
+        if (cell[q] >= 0)
+            atomicAdd(&cnt[cell[q]], sum[q]);
 }
 
 __global__ void k_flag(int ncell, int ref_ptcl, const int *__restrict__ cell_box,
@@ -127,8 +206,16 @@ __global__ void k_flag(int ncell, int ref_ptcl, const int *__restrict__ cell_box
 // neighbours inside a node's box.  Every parent pointer refers to a smaller cell
 // position or to the cell itself, so the root of a component is its first cell
 // and zones come out numbered in the order of their first cell, as the
-// reference numbers them.  The start points every cell at its smallest refine
-// face neighbour, which leaves short trees for the hooking pass.
+// reference numbers them.  The start points every cell at the end of the run of
+// refine cells behind it, up to CC_REACH cells along z, y or x, the smallest of the
+// three: a chain to the root is then 1/CC_REACH as long as from neighbour to
+// neighbour, and it is the chain's loads, one after the other, that the next
+// kernels wait for.  A pass that points every cell at its root follows, so that
+// the hooking finds most roots in one step.  Start, pass and hooking take 51 us on the
+// 2.1M cells of a 128^3 head with a million particles' refine cells, and 30 on the 262k
+// of a 64^3 one; neighbour chains hooked at once took 65 and 36.
+constexpr int CC_REACH = 8;
+
 __global__ void k_cc_init(int ncell, const int *__restrict__ cell_box,
                           const int *__restrict__ cell_node, const AmrNode *__restrict__ nodes,
                           const int *__restrict__ box, const int *__restrict__ pos_of_box,
@@ -143,18 +230,32 @@ __global__ void k_cc_init(int ncell, const int *__restrict__ cell_box,
         parent[c] = -1;
         return;
     }
-    const AmrNode N = nodes[cell_node[c]];
-    const long sy = N.rd[0], sz = (long)N.rd[0] * N.rd[1];
-    const long off[6] = {1, -1, sy, -sy, sz, -sz};
+    const AmrNode &N = nodes[cell_node[c]];
+    // a run ends at the ring of the node's box at the latest: what is loaded beyond a
+    // run's end is not used, and stays within the node's box
+    const int first = (int)(b - N.box_off);
+    const int off[3] = {N.rd[0] * N.rd[1], N.rd[0], 1};
     int m = c;
-    for (int e = 0; e < 6; e++)
+#pragma unroll
+    for (int e = 0; e < 3; e++)
     {
-        const long nb = b + off[e];
-        if (box[nb] != -1)
-            continue;
-        const int q = pos_of_box[nb];
-        if (q >= 0 && q < m)
-            m = q;
+        int st[CC_REACH], far = 0;
+#pragma unroll
+        for (int k = 0; k < CC_REACH; k++)
+            st[k] = (long)(k + 1) * off[e] <= first ? box[b - (long)(k + 1) * off[e]] : 0;
+        bool run = true;
+#pragma unroll
+        for (int k = 0; k < CC_REACH; k++)
+        {
+            run = run && st[k] == -1;
+            far += run ? 1 : 0;
+        }
+        if (far > 0)
+        {
+            const int q = pos_of_box[b - (long)far * off[e]];
+            if (q >= 0 && q < m)
+                m = q;
+        }
     }
     parent[c] = m;
 }
@@ -178,26 +279,42 @@ __device__ __forceinline__ int cc_find(int *parent, int x)
 
 // Joins each refine cell with its +x, +y and +z refine neighbours (every face
 // once): the larger root is hooked under the smaller one by compare-and-swap.
+// Neighbouring cells mostly ask for the same two roots; one lane of a warp does it
+// for all of them, since the swaps of one word run one after the other (the hooking of
+// the 64^3 head's cells: 17 us, 24 with a swap a face).
 __global__ void k_cc_hook(int ncell, const int *__restrict__ cell_box,
                           const int *__restrict__ cell_node, const AmrNode *__restrict__ nodes,
                           const int *__restrict__ box, const int *__restrict__ pos_of_box,
                           int *parent, int *__restrict__ flags)
 {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell || __ldcg(&parent[c]) < 0)
+    const bool on = c < ncell && __ldcg(&parent[c]) >= 0;
+    if (!__any_sync(0xffffffffu, on))
         return;
-    const AmrNode N = nodes[cell_node[c]];
-    const long b = cell_box[c];
-    const long off[3] = {1, N.rd[0], (long)N.rd[0] * N.rd[1]};
+    int q[3] = {-1, -1, -1};
+    if (on)
+    {
+        const AmrNode &N = nodes[cell_node[c]];
+        const long b = cell_box[c];
+        const long off[3] = {1, N.rd[0], (long)N.rd[0] * N.rd[1]};
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+            if (box[b + off[e]] == -1)
+                q[e] = pos_of_box[b + off[e]];
+    }
     for (int e = 0; e < 3; e++)
     {
-        const long nb = b + off[e];
-        if (box[nb] != -1)
+        int ra = 0, rb = 0;
+        if (q[e] >= 0)
+        {
+            ra = cc_find(parent, c);
+            rb = cc_find(parent, q[e]);
+        }
+        const unsigned long long pair =
+            (unsigned long long)(unsigned)max(ra, rb) << 32 | (unsigned)min(ra, rb);
+        const unsigned grp = __match_any_sync(0xffffffffu, pair);
+        if (ra == rb || (int)(threadIdx.x & 31) != __ffs(grp) - 1)
             continue;
-        const int q = pos_of_box[nb];
-        if (q < 0)
-            continue;
-        int ra = cc_find(parent, c), rb = cc_find(parent, q);
         int guard = 0;
         for (; guard < (1 << 10) && ra != rb; guard++)
         {
@@ -218,65 +335,120 @@ __global__ void k_cc_hook(int ncell, const int *__restrict__ cell_box,
     }
 }
 
-// Every refine cell points at its root.
-__global__ void k_cc_compress(int ncell, int *parent)
+// Every refine cell points towards its root.  A cell with nothing behind it on any axis
+// first takes the smallest parent of the cells before it: a round blob's lower corner is
+// a staircase of such cells (hundreds, each the root of what lies above it, which the
+// hooking would join one by one), and one step up a stair the way down goes on.
+__global__ void k_cc_compress(int ncell, const int *__restrict__ cell_box,
+                              const int *__restrict__ cell_node,
+                              const AmrNode *__restrict__ nodes, const int *__restrict__ box,
+                              const int *__restrict__ pos_of_box, int *parent)
 {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell || __ldcg(&parent[c]) < 0)
+    if (c >= ncell)
         return;
-    const int r = cc_find(parent, c);
+    const int p = __ldcg(&parent[c]);
+    if (p < 0)
+        return;
+    int start = p;
+    if (p == c)
+    {
+        const AmrNode &N = nodes[cell_node[c]];
+        const long b = cell_box[c];
+        const long off[3] = {1, N.rd[0], (long)N.rd[0] * N.rd[1]};
+        int q[3];
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+            q[e] = box[b + off[e]] == -1 ? pos_of_box[b + off[e]] : -1;
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+            if (q[e] >= 0)
+                start = min(start, __ldcg(&parent[q[e]]));
+        if (start == c)
+            return;
+        __stcg(&parent[c], start);
+    }
+    const int r = cc_find(parent, start);
     __stcg(&parent[c], r);
 }
 
-__global__ void k_cc_roots(int ncell, const int *__restrict__ parent, int *__restrict__ is_root,
-                           int *__restrict__ flagged)
+// After the last hook: every refine cell points at its root (the way there is not
+// rewritten: a cell's pointer is stored by its own thread only), and every block leaves
+// its numbers of roots and of refine cells.
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_cc_count(int ncell, int nblk, int *parent, int *__restrict__ cnt)
 {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell)
-        return;
-    is_root[c] = parent[c] == c ? 1 : 0;
-    flagged[c] = parent[c] >= 0 ? 1 : 0;
+    __shared__ int sh[2][SEL_WARPS];
+    const int c = blockIdx.x * SEL_THREADS + threadIdx.x;
+    int x = c < ncell ? __ldcg(&parent[c]) : -1;
+    const bool on = x >= 0;
+    if (on)
+    {
+        for (int guard = 0; guard < (1 << 20); guard++)
+        {
+            const int p = __ldcg(&parent[x]);
+            if (p == x)
+                break;
+            x = p;
+        }
+        __stcg(&parent[c], x);
+    }
+    int rank;
+    const int roots = sel_rank(on && x == c, sh[0], &rank);
+    const int cells = sel_rank(on, sh[1], &rank);
+    if (threadIdx.x == 0)
+    {
+        cnt[blockIdx.x] = roots;
+        cnt[nblk + blockIdx.x] = cells;
+    }
 }
 
-__global__ void k_gather_at(int m, const int *const *__restrict__ at, int *__restrict__ out)
+// Zone record of a level: [0, 6 nz) the boxes (min x y z, max x y z), [6 nz, 7 nz) the
+// cells, [7 nz, 7 nz + 2 nn) first zone and zones of every node of the parent level,
+// then the zones' first cells.
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_zone_roots(int ncell, int nz, int nn, const int *__restrict__ parent,
+                 const int *__restrict__ base, int *__restrict__ zrank, int *__restrict__ zone)
 {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < m)
-        out[q] = *at[q];
-}
-
-__global__ void k_zone_box_init(int nz, int *zone_box, int *zone_cells)
-{
-    int z = blockIdx.x * blockDim.x + threadIdx.x;
-    if (z >= nz)
+    __shared__ int sh[SEL_WARPS];
+    const int c = blockIdx.x * SEL_THREADS + threadIdx.x;
+    const bool root = c < ncell && parent[c] == c;
+    int rank;
+    sel_rank(root, sh, &rank);
+    if (!root)
         return;
+    const int z = base[blockIdx.x] + rank;
+    zrank[c] = z;
     for (int q = 0; q < 3; q++)
     {
-        zone_box[6 * z + q] = INT_MAX;
-        zone_box[6 * z + 3 + q] = INT_MIN;
+        zone[6 * z + q] = INT_MAX;
+        zone[6 * z + 3 + q] = INT_MIN;
     }
-    zone_cells[z] = 0;
+    zone[6 * nz + z] = 0;
+    zone[7 * nz + 2 * nn + z] = c;
 }
 
-// Zone ids: zrank (exclusive scan of roots over the level's cells) is the
-// child index of each root in the next level; inside a node the zone id is
+// Zone ids: zrank (the roots numbered in cell order) is the child index of each
+// root in the next level; inside a node the zone id is
 // the rank minus the node's first rank.  Statuses of refine cells become zone
 // ids, and refine cells are written in cell order to (zone, cell) pairs.
-__global__ void k_cc_label(int ncell, const int *__restrict__ cell_box,
-                           const int *__restrict__ cell_node, const AmrNode *__restrict__ nodes,
-                           const int *__restrict__ parent, const int *__restrict__ zrank,
-                           const int *__restrict__ slot, int *__restrict__ box,
-                           int *__restrict__ zone_box, int *__restrict__ zone_cells,
-                           const int *__restrict__ cell_xyz, unsigned *__restrict__ key,
-                           int *__restrict__ val)
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_cc_label(int ncell, int nz, const int *__restrict__ cell_box,
+               const int *__restrict__ cell_node, const AmrNode *__restrict__ nodes,
+               const int *__restrict__ parent, const int *__restrict__ zrank,
+               const int *__restrict__ base, int *__restrict__ box, int *__restrict__ zone,
+               const int *__restrict__ cell_xyz, unsigned *__restrict__ key,
+               int *__restrict__ val)
 {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell)
+    __shared__ int sh[SEL_WARPS];
+    const int c = blockIdx.x * SEL_THREADS + threadIdx.x;
+    const int r = c < ncell ? parent[c] : -1; // the root (parents are compressed)
+    int rank;
+    if (sel_rank(r >= 0, sh, &rank) == 0)
         return;
-    const int r = parent[c]; // the root (parents are compressed)
     const int zg = r >= 0 ? zrank[r] : -1;
     // lanes of one zone add their bounds and count once (a zone spans many cells)
-    const unsigned grp = __match_any_sync(__activemask(), zg);
+    const unsigned grp = __match_any_sync(0xffffffffu, zg);
     if (r < 0)
         return;
     const int x = cell_xyz[3 * c + 0], y = cell_xyz[3 * c + 1], z = cell_xyz[3 * c + 2];
@@ -286,36 +458,54 @@ __global__ void k_cc_label(int ncell, const int *__restrict__ cell_box,
               z1 = __reduce_max_sync(grp, z);
     if ((int)(threadIdx.x & 31) == __ffs(grp) - 1)
     {
-        atomicMin(&zone_box[6 * zg + 0], x0);
-        atomicMin(&zone_box[6 * zg + 1], y0);
-        atomicMin(&zone_box[6 * zg + 2], z0);
-        atomicMax(&zone_box[6 * zg + 3], x1);
-        atomicMax(&zone_box[6 * zg + 4], y1);
-        atomicMax(&zone_box[6 * zg + 5], z1);
-        atomicAdd(&zone_cells[zg], __popc(grp));
+        atomicMin(&zone[6 * zg + 0], x0);
+        atomicMin(&zone[6 * zg + 1], y0);
+        atomicMin(&zone[6 * zg + 2], z0);
+        atomicMax(&zone[6 * zg + 3], x1);
+        atomicMax(&zone[6 * zg + 4], y1);
+        atomicMax(&zone[6 * zg + 5], z1);
+        atomicAdd(&zone[6 * nz + zg], __popc(grp));
     }
-    const AmrNode N = nodes[cell_node[c]];
-    box[cell_box[c]] = zg - N.zone_base;
-    key[slot[c]] = (unsigned)zg;
-    val[slot[c]] = c;
+    const int slot = base[blockIdx.x] - nz + rank; // the scan has the zones before the cells
+    box[cell_box[c]] = zg - nodes[cell_node[c]].zone_base;
+    key[slot] = (unsigned)zg;
+    val[slot] = c;
 }
 
-__global__ void k_set_zone_base(int nn, AmrNode *nodes, const int *__restrict__ zrank, int nz)
+// First zone and zones of every node: the zones whose first cell is the node's.
+__global__ void k_set_zone_base(int nn, AmrNode *nodes, int nz, int *__restrict__ zone)
 {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nn)
         return;
-    int b = zrank[nodes[q].cell_off];
-    int e = q + 1 < nn ? zrank[nodes[q + 1].cell_off] : nz;
-    nodes[q].zone_base = b;
-    nodes[q].nzones = e - b;
+    const int *first = zone + 7 * nz + 2 * nn;
+    int at[2];
+    for (int e = 0; e < 2; e++)
+    {
+        int lo = 0, hi = nz;
+        if (q + e >= nn)
+            lo = nz;
+        const int cell = q + e < nn ? nodes[q + e].cell_off : 0;
+        while (lo < hi)
+        {
+            const int mid = (lo + hi) >> 1;
+            if (first[mid] < cell)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        at[e] = lo;
+    }
+    nodes[q].zone_base = at[0];
+    nodes[q].nzones = at[1] - at[0];
+    zone[7 * nz + 2 * q] = at[0];
+    zone[7 * nz + 2 * q + 1] = at[1] - at[0];
 }
 
 // Children: the j-th cell of zone z (cell order) spawns child cells
 // 8 j + (ii + 2 jj + 4 kk) of child node z (tree_construction.c:1634-1671).
 __global__ void k_child_cells(int nzc, const unsigned *__restrict__ zkey,
-                              const int *__restrict__ zval, const int *__restrict__ zone_start,
-                              const int *__restrict__ pcell_xyz, const AmrNode *__restrict__ cn,
+                              const int *__restrict__ zval, const int *__restrict__ pcell_xyz, const AmrNode *__restrict__ cn,
                               int *__restrict__ cell_box, int *__restrict__ cell_xyz,
                               int *__restrict__ cell_node)
 {
@@ -324,8 +514,8 @@ __global__ void k_child_cells(int nzc, const unsigned *__restrict__ zkey,
         return;
     int z = (int)zkey[q];
     int pc = zval[q];
-    int j = q - zone_start[z];
     const AmrNode N = cn[z];
+    int j = q - N.cell_off / 8;
     int px = 2 * pcell_xyz[3 * pc], py = 2 * pcell_xyz[3 * pc + 1], pz = 2 * pcell_xyz[3 * pc + 2];
     for (int sub = 0; sub < 8; sub++)
     {
@@ -350,31 +540,39 @@ __global__ void k_box_cells(int ncell, const int *__restrict__ cell_box, int *__
     pos_of_box[cell_box[c]] = c;
 }
 
-// Cells beyond the simulation box of a node that touches it (tree_construction.c:1745-1841).
-__global__ void k_box_simb(long total, int nn, const AmrNode *__restrict__ nodes,
-                           int *__restrict__ box)
+// Start of a level's box: status -4, or -5 beyond the simulation box of a node that
+// touches it (tree_construction.c:1745-1841; contact: the level has such a node), no
+// cell, no particles.
+__global__ void k_box_init(long total, int nn, const AmrNode *__restrict__ nodes, int contact,
+                           int *__restrict__ box, int *__restrict__ pos_of_box,
+                           int *__restrict__ cnt)
 {
     long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total)
         return;
-    const AmrNode N = nodes[find_node(nodes, nn, t, 2)];
-    if (!N.contact)
-        return;
-    long l = t - N.box_off;
-    int i = (int)(l % N.rd[0]), j = (int)((l / N.rd[0]) % N.rd[1]),
-        k = (int)(l / ((long)N.rd[0] * N.rd[1]));
-    const int top = 1 << N.lv;
-    const int g[3] = {i + N.ts[0], j + N.ts[1], k + N.ts[2]};
+    pos_of_box[t] = -1;
+    cnt[t] = 0;
     bool outside = false;
-    for (int a = 0; a < 3; a++)
+    if (contact)
     {
-        if (N.bmin[a] == 0 && g[a] < 0)
-            outside = true;
-        if (N.bmax[a] == top - 1 && g[a] >= top)
-            outside = true;
+        const AmrNode &N = nodes[find_node(nodes, nn, t, 2)];
+        if (N.contact)
+        {
+            const unsigned l = (unsigned)(t - N.box_off), rx = N.rd[0], ry = N.rd[1];
+            const unsigned row = l / rx, k = row / ry;
+            const int top = 1 << N.lv;
+            const int g[3] = {(int)(l - row * rx) + N.ts[0], (int)(row - k * ry) + N.ts[1],
+                              (int)k + N.ts[2]};
+            for (int a = 0; a < 3; a++)
+            {
+                if (N.bmin[a] == 0 && g[a] < 0)
+                    outside = true;
+                if (N.bmax[a] == top - 1 && g[a] >= top)
+                    outside = true;
+            }
+        }
     }
-    if (outside)
-        box[t] = -5;
+    box[t] = outside ? -5 : -4;
 }
 
 // Grid-point category from the 8 cells around the point (tree_construction.c:1935-2107):
@@ -405,68 +603,115 @@ __device__ __forceinline__ int classify_point(const int *box, long b, long sy, l
     return bder ? 2 : 1;
 }
 
-// Per node, the box grid points [bmin - ts, bmax - ts + 1]^3 in box order; fl
-// holds three flag arrays (interior | boundary | simulation boundary); interior
-// points are marked in the bricks of the conjugate-gradient order, if given.
-__global__ void k_classify(long total, int nn, const AmrNode *__restrict__ nodes,
-                           const int *__restrict__ box, int *__restrict__ fl,
-                           unsigned long long *__restrict__ bricks)
+// Place t of a level's classification range: its node (in *nd) and box grid
+// coordinates; false for the fill behind a node's last point (a node's range is whole
+// blocks of SEL_THREADS points).
+__device__ __forceinline__ bool class_point(const AmrNode *__restrict__ nodes, int nn, long t,
+                                            int *nd, int *ii, int *jj, int *kk)
 {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total)
-        return;
-    const AmrNode N = nodes[find_node(nodes, nn, t, 1)];
-    const int ex = N.bmax[0] - N.bmin[0] + 2, ey = N.bmax[1] - N.bmin[1] + 2;
-    long l = t - N.cls_off;
-    int ii = N.bmin[0] - N.ts[0] + (int)(l % ex);
-    int jj = N.bmin[1] - N.ts[1] + (int)((l / ex) % ey);
-    int kk = N.bmin[2] - N.ts[2] + (int)(l / ((long)ex * ey));
-    const long sy = N.rd[0], sz = (long)N.rd[0] * N.rd[1];
-    long b = N.box_off + ii + jj * sy + kk * sz;
-    int cat = classify_point(box, b, sy, sz, ii + N.ts[0], jj + N.ts[1], kk + N.ts[2], 1 << N.lv,
-                             N.contact);
-    if (bricks && cat == 1)
-        brick_mark(N, ii, jj, kk, bricks);
-    fl[t] = cat == 1;
-    fl[total + t] = cat == 2;
-    fl[2 * total + t] = cat == 3;
+    *nd = find_node(nodes, nn, t, 1);
+    const AmrNode &N = nodes[*nd];
+    const unsigned ex = N.bmax[0] - N.bmin[0] + 2, ey = N.bmax[1] - N.bmin[1] + 2,
+                   ez = N.bmax[2] - N.bmin[2] + 2;
+    const unsigned l = (unsigned)(t - N.cls_off), row = l / ex, k = row / ey;
+    *ii = N.bmin[0] - N.ts[0] + (int)(l - row * ex);
+    *jj = N.bmin[1] - N.ts[1] + (int)(row - k * ey);
+    *kk = N.bmin[2] - N.ts[2] + (int)k;
+    return k < ez;
 }
 
-__global__ void k_lists(long total, int nn, const AmrNode *__restrict__ nodes,
-                        const int *__restrict__ fl, const int *__restrict__ pos, int base1,
-                        int base2, int *__restrict__ intr, int *__restrict__ bdry,
-                        int *__restrict__ simb, int *__restrict__ intr_node,
-                        int *__restrict__ bdry_node, int *__restrict__ simb_node)
+// Per node, the box grid points [bmin - ts, bmax - ts + 1]^3 in box order: cat holds a
+// point's category, cnt three lists (interior | boundary | simulation boundary) of the
+// blocks' numbers; interior points are marked in the bricks of the conjugate-gradient
+// order, if given.
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_classify(int nblk, int nn, const AmrNode *__restrict__ nodes, const int *__restrict__ box,
+               unsigned char *__restrict__ cat, int *__restrict__ cnt,
+               unsigned long long *__restrict__ bricks)
 {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total)
-        return;
-    int cat = fl[t] ? 0 : fl[total + t] ? 1 : fl[2 * total + t] ? 2 : -1;
-    if (cat < 0)
-        return;
-    int nd = find_node(nodes, nn, t, 1);
-    const AmrNode N = nodes[nd];
-    const int ex = N.bmax[0] - N.bmin[0] + 2, ey = N.bmax[1] - N.bmin[1] + 2;
-    long l = t - N.cls_off;
-    int ii = N.bmin[0] - N.ts[0] + (int)(l % ex);
-    int jj = N.bmin[1] - N.ts[1] + (int)((l / ex) % ey);
-    int kk = N.bmin[2] - N.ts[2] + (int)(l / ((long)ex * ey));
-    int g = (int)grid_index(N, ii, jj, kk);
-    int p = pos[cat * total + t];
-    if (cat == 0)
+    __shared__ int sh[3][SEL_WARPS];
+    const long t = (long)blockIdx.x * SEL_THREADS + threadIdx.x;
+    int nd, ii, jj, kk, c = 0;
+    if (class_point(nodes, nn, t, &nd, &ii, &jj, &kk))
     {
+        const AmrNode &N = nodes[nd];
+        const long sy = N.rd[0], sz = (long)N.rd[0] * N.rd[1];
+        const long b = N.box_off + ii + jj * sy + kk * sz;
+        c = classify_point(box, b, sy, sz, ii + N.ts[0], jj + N.ts[1], kk + N.ts[2], 1 << N.lv,
+                           N.contact);
+        if (bricks && c == 1)
+            brick_mark(N, ii, jj, kk, bricks);
+    }
+    cat[t] = (unsigned char)c;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+    {
+        int rank;
+        const int m = sel_rank(c == q + 1, sh[q], &rank);
+        if (threadIdx.x == 0)
+            cnt[q * nblk + blockIdx.x] = m;
+    }
+}
+
+// Every node's first place in the three lists (of the scan over all three), the places'
+// total, and, with the conjugate-gradient order, the nodes' first rows and the rows' total.
+__global__ void k_level_starts(int nn, const AmrNode *__restrict__ nodes, int nblk,
+                               const int *__restrict__ cnt, const int *__restrict__ pos,
+                               const int *__restrict__ brick_base, int nbricks,
+                               int *__restrict__ out)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nn)
+        return;
+    const long b = nodes[q].cls_off / SEL_THREADS;
+    for (int c = 0; c < 3; c++)
+        out[c * nn + q] = pos[(long)c * nblk + b];
+    if (brick_base)
+        out[3 * nn + 1 + q] = brick_base[nodes[q].brick_off];
+    if (q == 0)
+    {
+        out[3 * nn] = pos[3L * nblk - 1] + cnt[3L * nblk - 1];
+        if (brick_base)
+            out[4 * nn + 1] = brick_base[nbricks - 1] + brick_base[2L * nbricks - 1];
+    }
+}
+
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_lists(int nblk, int nn, const AmrNode *__restrict__ nodes,
+            const unsigned char *__restrict__ cat, const int *__restrict__ pos, int base1,
+            int base2, int *__restrict__ intr, int *__restrict__ bdry, int *__restrict__ simb,
+            int *__restrict__ intr_node, int *__restrict__ bdry_node, int *__restrict__ simb_node)
+{
+    __shared__ int sh[3][SEL_WARPS];
+    const long t = (long)blockIdx.x * SEL_THREADS + threadIdx.x;
+    const int c = cat[t];
+    int rank[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        sel_rank(c == q + 1, sh[q], &rank[q]);
+    if (c == 0)
+        return;
+    int nd, ii, jj, kk;
+    class_point(nodes, nn, t, &nd, &ii, &jj, &kk);
+    const int g = (int)grid_index(nodes[nd], ii, jj, kk);
+    const int *at = pos + blockIdx.x;
+    if (c == 1)
+    {
+        const int p = at[0] + rank[0];
         intr[p] = g;
         intr_node[p] = nd;
     }
-    else if (cat == 1)
+    else if (c == 2)
     {
-        bdry[p - base1] = g;
-        bdry_node[p - base1] = nd;
+        const int p = at[nblk] + rank[1] - base1;
+        bdry[p] = g;
+        bdry_node[p] = nd;
     }
     else
     {
-        simb[p - base2] = g;
-        simb_node[p - base2] = nd;
+        const int p = at[2L * nblk] + rank[2] - base2;
+        simb[p] = g;
+        simb_node[p] = nd;
     }
 }
 
@@ -526,25 +771,27 @@ static bool read_ints(qz_sim *s, const int *dsrc, long count, int *out)
     return true;
 }
 
-// Reads *at[q] for every device address of the list (one launch, one read-back).
-static bool read_at(qz_sim *s, const std::vector<const int *> &at, int *out)
+// Waits for what the stream's kernels wrote to h_small.
+static bool wait_small(qz_sim *s)
+{
+    return check_cuda(cudaGetLastError(), "read back") &&
+           check_cuda(cudaStreamSynchronize(s->stream), "read back sync");
+}
+
+// Reads *at[q] for up to READ_FEW device addresses: one launch that writes to the host, one
+// wait (the addresses travel as the kernel's argument: no copy either way).
+static bool read_few(qz_sim *s, const std::vector<const int *> &at, int *out)
 {
     const int m = (int)at.size();
-    if (m == 0)
-        return true;
-    if (!s->gather_idx.ensure(s->mem, 3L * m) || !ensure_small(s, 2L * m))
-    {
-        set_error("gather buffer");
+    ReadList L{};
+    if (m > READ_FEW || !ensure_small(s, READ_FEW))
         return false;
-    }
-    memcpy(s->h_small, at.data(), m * sizeof(const int *));
-    if (!check_cuda(cudaMemcpyAsync(s->gather_idx.p, s->h_small, m * sizeof(const int *),
-                                    cudaMemcpyHostToDevice, s->stream),
-                    "gather h2d"))
+    std::copy(at.begin(), at.end(), L.at);
+    launch(s, QZ_PROF_TREE, 8.0 * m, k_read_few, dim3(1), dim3(READ_FEW), m, L, s->h_small);
+    if (!wait_small(s))
         return false;
-    launch(s, QZ_PROF_TREE, 16.0 * m, k_gather_at, dim3(blocks_for(m, 256)), dim3(256), m,
-           (const int *const *)s->gather_idx.p, s->gather_idx.p + 2L * m);
-    return read_ints(s, s->gather_idx.p + 2L * m, m, out);
+    memcpy(out, s->h_small, m * sizeof(int));
+    return true;
 }
 
 static bool upload_nodes(qz_sim *s, AmrLevel &L)
@@ -593,8 +840,6 @@ void amr_free(qz_sim *s)
     s->amr_tmp.release(s->mem);
     s->amr_tmp2.release(s->mem);
     s->zone_box.release(s->mem);
-    s->zone_cells.release(s->mem);
-    s->gather_idx.release(s->mem);
     s->seg_mass.release(s->mem);
     s->cgr_halo.release(s->mem);
     s->cgr_sums.release(s->mem);
@@ -728,11 +973,9 @@ int amr_build(qz_sim *s)
     const long n = s->n;
     const int levels = (int)s->amr.size();
     AmrLevel &H = s->amr[0];
-    // head statuses (initialization.c:95-110): -5 on the ghost ring, -3 inside
-    launch(s, QZ_PROF_TREE, 4.0 * H.box_total, k_fill_int, dim3(blocks_for(H.box_total, 256)),
-           dim3(256), H.box_total, H.box.p, -5);
-    launch(s, QZ_PROF_TREE, 8.0 * H.cell_total, k_box_cells, dim3(blocks_for(H.cell_total, 256)),
-           dim3(256), H.cell_total, H.cell_box.p, H.box.p, H.pos_of_box.p);
+    const int B = (1 << s->L) + 2;
+    launch(s, QZ_PROF_TREE, 8.0 * H.box_total, k_head_box, dim3(blocks_for((long)B * B, 256), B),
+           dim3(256), B, H.box.p, H.cnt.p);
     cudaMemsetAsync(s->node_of[0].p, 0, (n > 0 ? n : 1) * sizeof(int), s->stream);
     s->amr_nlev = 1;
     for (int l = 1; l < levels; l++)
@@ -742,37 +985,38 @@ int amr_build(qz_sim *s)
         AmrLevel &P = s->amr[l];
         if (P.nnodes == 0)
             break;
-        cudaMemsetAsync(P.cnt.p, 0, P.box_total * sizeof(int), s->stream);
         if (n > 0)
-            launch(s, QZ_PROF_TREE, 28.0 * n, k_count, dim3(blocks_for(n, 256)), dim3(256), n,
-                   s->node_of[l].p, P.nodes.p, s->x, s->y, s->z, P.cnt.p, s->flags);
+            launch(s, QZ_PROF_TREE, 28.0 * n, k_count, dim3(blocks_for(n, COUNT_THREADS * COUNT_ITEMS)),
+                   dim3(COUNT_THREADS), n, s->node_of[l].p, P.nodes.p, s->x, s->y, s->z, P.cnt.p,
+                   s->flags);
         const int nc = P.cell_total;
         launch(s, QZ_PROF_TREE, 12.0 * nc, k_flag, dim3(blocks_for(nc, 256)), dim3(256), nc,
                s->cfg.ref_ptcl, P.cell_box.p, P.cell_node.p, P.nodes.p, P.cnt.p, P.box.p);
-        // union-find over the refine cells: parent | is_root | zone rank | flagged | slot
-        if (!s->amr_tmp.ensure(s->mem, 5L * nc + 8))
+        // union-find over the refine cells: parent | zone rank | blocks' roots and refine
+        // cells | their scan
+        const int ncb = blocks_for(nc, SEL_THREADS);
+        if (!s->amr_tmp.ensure(s->mem, 2L * nc + 4L * ncb))
         {
             set_error("amr scratch");
             return QZ_FAILURE;
         }
-        int *parent = s->amr_tmp.p, *isroot = parent + nc, *zrank = isroot + nc,
-            *flagged = zrank + nc, *slot = flagged + nc;
+        int *parent = s->amr_tmp.p, *zrank = parent + nc, *zcnt = zrank + nc, *zpos = zcnt + 2L * ncb;
         launch(s, QZ_PROF_TREE, 36.0 * nc, k_cc_init, dim3(blocks_for(nc, 256)), dim3(256), nc,
+               P.cell_box.p, P.cell_node.p, P.nodes.p, P.box.p, P.pos_of_box.p, parent);
+        launch(s, QZ_PROF_TREE, 8.0 * nc, k_cc_compress, dim3(blocks_for(nc, 256)), dim3(256), nc,
                P.cell_box.p, P.cell_node.p, P.nodes.p, P.box.p, P.pos_of_box.p, parent);
         launch(s, QZ_PROF_TREE, 32.0 * nc, k_cc_hook, dim3(blocks_for(nc, 256)), dim3(256), nc,
                P.cell_box.p, P.cell_node.p, P.nodes.p, P.box.p, P.pos_of_box.p, parent,
                s->flags);
-        launch(s, QZ_PROF_TREE, 8.0 * nc, k_cc_compress, dim3(blocks_for(nc, 256)), dim3(256), nc,
-               parent);
-        launch(s, QZ_PROF_TREE, 12.0 * nc, k_cc_roots, dim3(blocks_for(nc, 256)), dim3(256), nc,
-               parent, isroot, flagged);
-        if (scan_exclusive(s, isroot, zrank, nc) || scan_exclusive(s, flagged, slot, nc))
+        launch(s, QZ_PROF_TREE, 8.0 * nc, k_cc_count, dim3(ncb), dim3(SEL_THREADS), nc, ncb, parent,
+               zcnt);
+        if (scan_exclusive(s, zcnt, zpos, 2L * ncb))
             return QZ_FAILURE;
-        // zones = last rank + last root flag; refine cells = last slot + last flag
-        int t[4];
-        if (!read_at(s, {zrank + nc - 1, isroot + nc - 1, slot + nc - 1, flagged + nc - 1}, t))
+        // zones, then zones and refine cells (the last block's place and number)
+        int t[3];
+        if (!read_few(s, {zpos + ncb, zpos + 2L * ncb - 1, zcnt + 2L * ncb - 1}, t))
             return QZ_FAILURE;
-        const int nz = t[0] + t[1], nzc = t[2] + t[3];
+        const int nz = t[0], nzc = t[1] + t[2] - nz;
         if (nz == 0)
         {
             for (auto &nd : P.h)
@@ -780,18 +1024,19 @@ int amr_build(qz_sim *s)
             upload_nodes(s, P);
             break;
         }
-        if (!s->zone_box.ensure(s->mem, 6L * nz) || !s->zone_cells.ensure(s->mem, nz) || !ensure_sort(s, nzc))
+        const long zinfo = 7L * nz + 2L * P.nnodes;
+        if (!s->zone_box.ensure(s->mem, zinfo + nz) || !ensure_sort(s, nzc))
         {
             set_error("zone buffers");
             return QZ_FAILURE;
         }
+        launch(s, QZ_PROF_TREE, 4.0 * nc, k_zone_roots, dim3(ncb), dim3(SEL_THREADS), nc, nz,
+               P.nnodes, parent, zpos, zrank, s->zone_box.p);
         launch(s, QZ_PROF_TREE, 4.0 * P.nnodes, k_set_zone_base, dim3(blocks_for(P.nnodes, 128)),
-               dim3(128), P.nnodes, P.nodes.p, zrank, nz);
-        launch(s, QZ_PROF_TREE, 28.0 * nz, k_zone_box_init, dim3(blocks_for(nz, 256)), dim3(256),
-               nz, s->zone_box.p, s->zone_cells.p);
-        launch(s, QZ_PROF_TREE, 48.0 * nc, k_cc_label, dim3(blocks_for(nc, 256)), dim3(256), nc,
-               P.cell_box.p, P.cell_node.p, P.nodes.p, parent, zrank, slot, P.box.p,
-               s->zone_box.p, s->zone_cells.p, P.cell_xyz.p, s->sort.k0, s->sort.v0);
+               dim3(128), P.nnodes, P.nodes.p, nz, s->zone_box.p);
+        launch(s, QZ_PROF_TREE, 48.0 * nc, k_cc_label, dim3(ncb), dim3(SEL_THREADS), nc, nz,
+               P.cell_box.p, P.cell_node.p, P.nodes.p, parent, zrank, zpos + ncb, P.box.p,
+               s->zone_box.p, P.cell_xyz.p, s->sort.k0, s->sort.v0);
         // zone cells in (zone, cell position) order: a stable sort on the zone id
         int zbits = 1;
         while ((1L << zbits) < nz)
@@ -800,18 +1045,14 @@ int amr_build(qz_sim *s)
         int *zv;
         if (radix_sort_pairs(s, nzc, zbits, &zk, &zv))
             return QZ_FAILURE;
-        std::vector<int> zbox(6L * nz), zcells(nz);
-        std::vector<AmrNode> pnodes(P.nnodes);
-        if (!read_ints(s, s->zone_box.p, 6L * nz, zbox.data()) ||
-            !read_ints(s, s->zone_cells.p, nz, zcells.data()) ||
-            !check_cuda(cudaMemcpyAsync(pnodes.data(), P.nodes.p, P.nnodes * sizeof(AmrNode),
-                                        cudaMemcpyDeviceToHost, s->stream), "nodes d2h") ||
-            !check_cuda(cudaStreamSynchronize(s->stream), "nodes d2h sync"))
+        std::vector<int> zbox(zinfo);
+        if (!read_ints(s, s->zone_box.p, zinfo, zbox.data()))
             return QZ_FAILURE;
+        const int *zcells = &zbox[6L * nz];
         for (int q = 0; q < P.nnodes; q++)
         {
-            P.h[q].zone_base = pnodes[q].zone_base;
-            P.h[q].nzones = pnodes[q].nzones;
+            P.h[q].zone_base = zbox[7L * nz + 2L * q];
+            P.h[q].nzones = zbox[7L * nz + 2L * q + 1];
         }
         // ---- child level geometry (host) ---------------------------------------------
         AmrLevel &C = s->amr[l + 1];
@@ -821,7 +1062,7 @@ int amr_build(qz_sim *s)
         int cell_total = 0;
         const int clv = P.h[0].lv + 1;
         const int top = 1 << clv;
-        std::vector<int> zstart(nz);
+        int contact = 0;
         for (int q = 0; q < P.nnodes; q++)
             for (int zz = 0; zz < P.h[q].nzones; zz++)
             {
@@ -837,19 +1078,19 @@ int amr_build(qz_sim *s)
                     N.rd[a] = dim + s->cfg.box_extra;
                     N.ts[a] = N.bmin[a] - (N.rd[a] - dim) / 2;
                     if (N.bmin[a] == 0 || N.bmax[a] == top - 1)
-                        N.contact = 1;
+                        N.contact = contact = 1;
                 }
                 N.box_off = box_total;
                 box_total += (long)N.rd[0] * N.rd[1] * N.rd[2];
                 N.grid_off = grid_total;
                 grid_total += (long)(N.rd[0] + 1) * (N.rd[1] + 1) * (N.rd[2] + 1);
-                zstart[z] = cell_total / 8;
                 N.cell_off = cell_total;
                 N.ncells = 8 * zcells[z];
                 cell_total += N.ncells;
                 N.cls_off = cls_total;
                 cls_total += (long)(N.bmax[0] - N.bmin[0] + 2) * (N.bmax[1] - N.bmin[1] + 2) *
                              (N.bmax[2] - N.bmin[2] + 2);
+                cls_total = (cls_total + SEL_THREADS - 1) / SEL_THREADS * SEL_THREADS;
             }
         C.box_total = box_total;
         C.grid_total = grid_total;
@@ -860,65 +1101,45 @@ int amr_build(qz_sim *s)
         cg_brick_layout(C);
         if (order && cg_brick_masks(s, C, &bricks))
             return QZ_FAILURE;
+        // blocks' numbers of points of each category | their scan | the points' categories
+        const int nblk = (int)(cls_total / SEL_THREADS);
         if (!C.box.ensure(s->mem, box_total) || !C.cnt.ensure(s->mem, box_total) ||
             !C.pos_of_box.ensure(s->mem, box_total) || !C.cell_box.ensure(s->mem, cell_total) ||
             !C.cell_xyz.ensure(s->mem, 3L * cell_total) || !C.cell_node.ensure(s->mem, cell_total) ||
-            !s->amr_tmp2.ensure(s->mem, std::max((long)nz, 6L * cls_total + 8)))
+            !s->amr_tmp2.ensure(s->mem, 6L * nblk + cls_total / 4))
         {
             set_error("child level buffers");
             return QZ_FAILURE;
         }
         if (!upload_nodes(s, C))
             return QZ_FAILURE;
-        int *dzstart = s->amr_tmp2.p;
-        if (!ensure_small(s, nz))
-            return QZ_FAILURE;
-        memcpy(s->h_small, zstart.data(), nz * sizeof(int));
-        if (!check_cuda(cudaMemcpyAsync(dzstart, s->h_small, nz * sizeof(int),
-                                        cudaMemcpyHostToDevice, s->stream),
-                        "zone start") ||
-            !check_cuda(cudaStreamSynchronize(s->stream), "zone start sync"))
-            return QZ_FAILURE;
         launch(s, QZ_PROF_TREE, 40.0 * nzc, k_child_cells, dim3(blocks_for(nzc, 256)), dim3(256),
-               nzc, zk, zv, dzstart, P.cell_xyz.p, C.nodes.p, C.cell_box.p, C.cell_xyz.p,
+               nzc, zk, zv, P.cell_xyz.p, C.nodes.p, C.cell_box.p, C.cell_xyz.p,
                C.cell_node.p);
-        launch(s, QZ_PROF_TREE, 4.0 * box_total, k_fill_int, dim3(blocks_for(box_total, 256)),
-               dim3(256), box_total, C.box.p, -4);
-        launch(s, QZ_PROF_TREE, 4.0 * box_total, k_fill_int, dim3(blocks_for(box_total, 256)),
-               dim3(256), box_total, C.pos_of_box.p, -1);
+        launch(s, QZ_PROF_TREE, 12.0 * box_total, k_box_init, dim3(blocks_for(box_total, 256)),
+               dim3(256), box_total, C.nnodes, C.nodes.p, contact, C.box.p, C.pos_of_box.p, C.cnt.p);
         launch(s, QZ_PROF_TREE, 8.0 * cell_total, k_box_cells, dim3(blocks_for(cell_total, 256)),
                dim3(256), cell_total, C.cell_box.p, C.box.p, C.pos_of_box.p);
-        launch(s, QZ_PROF_TREE, 4.0 * box_total, k_box_simb, dim3(blocks_for(box_total, 256)),
-               dim3(256), box_total, C.nnodes, C.nodes.p, C.box.p);
         // grid-point lists
-        int *fl = s->amr_tmp2.p, *pos = fl + 3 * cls_total;
-        launch(s, QZ_PROF_TREE, 32.0 * cls_total, k_classify, dim3(blocks_for(cls_total, 256)),
-               dim3(256), cls_total, C.nnodes, C.nodes.p, C.box.p, fl, bricks);
-        if (scan_exclusive(s, fl, pos, 3 * cls_total) || (order && cg_brick_scan(s, C)))
+        int *pcnt = s->amr_tmp2.p, *pos = pcnt + 3L * nblk;
+        unsigned char *cat = (unsigned char *)(pos + 3L * nblk);
+        launch(s, QZ_PROF_TREE, 33.0 * cls_total, k_classify, dim3(nblk), dim3(SEL_THREADS), nblk,
+               C.nnodes, C.nodes.p, C.box.p, cat, pcnt, bricks);
+        if (scan_exclusive(s, pcnt, pos, 3L * nblk) || (order && cg_brick_scan(s, C)))
             return QZ_FAILURE;
-        // scan values at every node's range start in each category, and the totals; the
-        // same of the nodes' rows in the conjugate-gradient order
-        std::vector<const int *> at;
-        for (int cat = 0; cat < 3; cat++)
-            for (int q = 0; q < nz; q++)
-                at.push_back(pos + cat * cls_total + C.h[q].cls_off);
-        at.push_back(pos + 3 * cls_total - 1);
-        at.push_back(fl + 3 * cls_total - 1);
+        if (!ensure_small(s, 4L * nz + 2))
+            return QZ_FAILURE;
+        launch(s, QZ_PROF_TREE, 32.0 * nz, k_level_starts, dim3(blocks_for(nz, 128)), dim3(128), nz,
+               C.nodes.p, nblk, pcnt, pos, order ? s->brick_base.p : nullptr, (int)C.brick_total,
+               s->h_small);
+        if (!wait_small(s))
+            return QZ_FAILURE;
+        const std::vector<int> sv(s->h_small, s->h_small + (order ? 4L * nz + 2 : 3L * nz + 1));
+        const int total_all = sv[3 * nz];
         if (order)
         {
-            for (int q = 0; q < nz; q++)
-                at.push_back(s->brick_base.p + C.h[q].brick_off);
-            at.push_back(s->brick_base.p + C.brick_total - 1);
-            at.push_back(s->brick_base.p + 2 * C.brick_total - 1);
-        }
-        std::vector<int> sv(at.size());
-        if (!read_at(s, at, sv.data()))
-            return QZ_FAILURE;
-        const int total_all = sv[3 * nz] + sv[3 * nz + 1];
-        if (order)
-        {
-            const int *rv = &sv[3 * nz + 2];
-            C.row_total = rv[nz] + rv[nz + 1];
+            const int *rv = &sv[3 * nz + 1];
+            C.row_total = rv[nz];
             for (int q = 0; q < nz; q++)
             {
                 C.h[q].row_off = rv[q];
@@ -951,9 +1172,8 @@ int amr_build(qz_sim *s)
             set_error("grid lists");
             return QZ_FAILURE;
         }
-        launch(s, QZ_PROF_TREE, 24.0 * cls_total, k_lists, dim3(blocks_for(cls_total, 256)),
-               dim3(256), cls_total, C.nnodes, C.nodes.p, fl, pos, start(1, 0), start(2, 0),
-               C.intr.p, C.bdry.p, C.simb.p, C.intr_node.p, C.bdry_node.p, C.simb_node.p);
+        launch(s, QZ_PROF_TREE, 9.0 * cls_total, k_lists, dim3(nblk), dim3(SEL_THREADS), nblk,
+               C.nnodes, C.nodes.p, cat, pos, start(1, 0), start(2, 0), C.intr.p, C.bdry.p, C.simb.p, C.intr_node.p, C.bdry_node.p, C.simb_node.p);
         if (!upload_nodes(s, C))
             return QZ_FAILURE;
         if (n > 0)
@@ -971,29 +1191,51 @@ int amr_build(qz_sim *s)
 
 
 // ---- deposit on refinement levels ------------------------------------------------------
-__global__ void k_lvl_keys(long n, const int *__restrict__ node_of, const AmrNode *__restrict__ nodes,
-                           const double *__restrict__ x, const double *__restrict__ y,
-                           const double *__restrict__ z, const int *__restrict__ slot,
-                           unsigned *__restrict__ keys, int *__restrict__ vals)
+struct LevelNodes {
+    const int *node_of[AMR_MAX_LEVELS];
+};
+
+// Particles of a block's SEL_THREADS that lie on each of the nl levels below the head.
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_lvl_count(long n, int nl, const __grid_constant__ LevelNodes L, int *__restrict__ cnt)
 {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    int nd = node_of[i];
-    if (nd < 0)
-        return;
-    const AmrNode N = nodes[nd];
-    const double sc = (double)(1 << N.lv);
-    int cx = (int)(x[i] * sc), cy = (int)(y[i] * sc), cz = (int)(z[i] * sc);
-    keys[slot[i]] = (unsigned)(N.box_off + box_index(N, cx, cy, cz));
-    vals[slot[i]] = (int)i;
+    const long i = (long)blockIdx.x * SEL_THREADS + threadIdx.x;
+    for (int l = 0; l < nl; l++)
+    {
+        const int m = __syncthreads_count(i < n && L.node_of[1 + l][i] >= 0);
+        if (threadIdx.x == 0)
+            cnt[(long)l * gridDim.x + blockIdx.x] = m;
+        if (m == 0)
+        {
+            // none on this level, so none below it
+            for (l++; l < nl; l++)
+                if (threadIdx.x == 0)
+                    cnt[(long)l * gridDim.x + blockIdx.x] = 0;
+        }
+    }
 }
 
-__global__ void k_in_level(long n, const int *__restrict__ node_of, int *__restrict__ flag)
+// Cells and numbers of the level's particles, in particle order (base: the scanned counts
+// of the level's blocks).
+__global__ void __launch_bounds__(SEL_THREADS)
+    k_lvl_keys(long n, const int *__restrict__ node_of, const AmrNode *__restrict__ nodes,
+               const double *__restrict__ x, const double *__restrict__ y,
+               const double *__restrict__ z, const int *__restrict__ base,
+               unsigned *__restrict__ keys, int *__restrict__ vals)
 {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
-        flag[i] = node_of[i] >= 0 ? 1 : 0;
+    __shared__ int sh[SEL_WARPS];
+    const long i = (long)blockIdx.x * SEL_THREADS + threadIdx.x;
+    const int nd = i < n ? node_of[i] : -1;
+    int rank;
+    sel_rank(nd >= 0, sh, &rank);
+    if (nd < 0)
+        return;
+    const AmrNode &N = nodes[nd];
+    const double sc = (double)(1 << N.lv);
+    int cx = (int)(x[i] * sc), cy = (int)(y[i] * sc), cz = (int)(z[i] * sc);
+    const int slot = base[blockIdx.x] - base[0] + rank;
+    keys[slot] = (unsigned)(N.box_off + box_index(N, cx, cy, cz));
+    vals[slot] = (int)i;
 }
 
 // CIC corner sums with the branch weights (grid_density.c:166-245):
@@ -1195,29 +1437,51 @@ int deposit_segments(qz_sim *s, long m, int bits, int *cell_seg, long ncells_box
 int amr_deposit(qz_sim *s)
 {
     const long n = s->n;
-    for (int l = 1; l < s->amr_nlev; l++)
+    int nl = 0; // levels below the head
+    while (nl + 1 < s->amr_nlev && s->amr[nl + 1].nnodes > 0)
+        nl++;
+    if (nl == 0)
+        return QZ_SUCCESS;
+    // the levels' particles counted and read back together: one wait, not one a level
+    const int nb = blocks_for(n, SEL_THREADS);
+    if (!s->amr_tmp.ensure(s->mem, 2L * nl * nb) || !ensure_sort(s, n))
+    {
+        set_error("level deposit buffers");
+        return QZ_FAILURE;
+    }
+    int *cnt = s->amr_tmp.p, *base = cnt + (long)nl * nb;
+    LevelNodes LN{};
+    std::vector<const int *> at;
+    for (int l = 1; l <= nl; l++)
+    {
+        LN.node_of[l] = s->node_of[l].p;
+        at.push_back(base + (long)(l - 1) * nb);
+    }
+    at.push_back(base + (long)nl * nb - 1);
+    at.push_back(cnt + (long)nl * nb - 1);
+    std::vector<int> first(nl + 2);
+    if (n > 0)
+    {
+        launch(s, QZ_PROF_DEPOSIT, 4.0 * n * nl, k_lvl_count, dim3(nb), dim3(SEL_THREADS), n, nl, LN,
+               cnt);
+        if (scan_exclusive(s, cnt, base, (long)nl * nb) || !read_few(s, at, first.data()))
+            return QZ_FAILURE;
+        first[nl] += first[nl + 1];
+    }
+    for (int l = 1; l <= nl; l++)
     {
         AmrLevel &L = s->amr[l];
-        if (L.nnodes == 0)
-            break;
-        if (!L.gd.ensure(s->mem, L.grid_total) || !L.cell_seg.ensure(s->mem, L.box_total) ||
-            !s->amr_tmp.ensure(s->mem, 2 * n + 2) || !ensure_sort(s, n))
+        if (!L.gd.ensure(s->mem, L.grid_total) || !L.cell_seg.ensure(s->mem, L.box_total))
         {
             set_error("level deposit buffers");
             return QZ_FAILURE;
         }
         L.d = L.gd.p;
-        int *flag = s->amr_tmp.p, *slot = flag + n;
-        launch(s, QZ_PROF_DEPOSIT, 8.0 * n, k_in_level, dim3(blocks_for(n, 256)), dim3(256), n,
-               s->node_of[l].p, flag);
-        if (scan_exclusive(s, flag, slot, n))
-            return QZ_FAILURE;
-        int t[2];
-        if (!read_at(s, {slot + n - 1, flag + n - 1}, t))
-            return QZ_FAILURE;
-        const long m = t[0] + t[1];
-        launch(s, QZ_PROF_DEPOSIT, 44.0 * n, k_lvl_keys, dim3(blocks_for(n, 256)), dim3(256), n,
-               s->node_of[l].p, L.nodes.p, s->x, s->y, s->z, slot, s->sort.k0, s->sort.v0);
+        const long m = first[l] - first[l - 1];
+        if (n > 0)
+            launch(s, QZ_PROF_DEPOSIT, 44.0 * n, k_lvl_keys, dim3(nb), dim3(SEL_THREADS), n,
+                   s->node_of[l].p, L.nodes.p, s->x, s->y, s->z, base + (long)(l - 1) * nb,
+                   s->sort.k0, s->sort.v0);
         int bits = 1;
         while ((1L << bits) < L.box_total)
             bits++;
@@ -1256,19 +1520,32 @@ int amr_deposit(qz_sim *s)
         launch(s, QZ_PROF_DEPOSIT, 8.0 * NM_PARTS * L.nnodes, k_node_mass,
                dim3(blocks_for(L.nnodes, 128)), dim3(128), L.nnodes, L.nodes.p, s->seg_start,
                L.mass_part.p, L.mass_range.p);
-        std::vector<AmrNode> tmp(L.nnodes);
-        if (!check_cuda(cudaMemcpyAsync(tmp.data(), L.nodes.p, L.nnodes * sizeof(AmrNode),
-                                        cudaMemcpyDeviceToHost, s->stream), "nodes d2h") ||
-            !check_cuda(cudaStreamSynchronize(s->stream), "nodes d2h sync"))
-            return QZ_FAILURE;
-        for (int q = 0; q < L.nnodes; q++)
-        {
-            L.h[q].mass = tmp[q].mass;
-            L.h[q].nptcl = tmp[q].nptcl;
-        }
         if (!check_cuda(cudaGetLastError(), "level deposit"))
             return QZ_FAILURE;
     }
+    // the host's copies of the masses, all levels with one wait
+    long nn = 0;
+    for (int l = 1; l <= nl; l++)
+        nn += s->amr[l].nnodes;
+    std::vector<AmrNode> tmp(nn);
+    long q0 = 0;
+    for (int l = 1; l <= nl; l++)
+    {
+        const AmrLevel &L = s->amr[l];
+        if (!check_cuda(cudaMemcpyAsync(&tmp[q0], L.nodes.p, L.nnodes * sizeof(AmrNode),
+                                        cudaMemcpyDeviceToHost, s->stream), "nodes d2h"))
+            return QZ_FAILURE;
+        q0 += L.nnodes;
+    }
+    if (!check_cuda(cudaStreamSynchronize(s->stream), "nodes d2h sync"))
+        return QZ_FAILURE;
+    q0 = 0;
+    for (int l = 1; l <= nl; l++)
+        for (AmrNode &N : s->amr[l].h)
+        {
+            N.mass = tmp[q0].mass;
+            N.nptcl = tmp[q0++].nptcl;
+        }
     return QZ_SUCCESS;
 }
 

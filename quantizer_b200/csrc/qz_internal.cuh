@@ -616,9 +616,7 @@ struct qz_sim {
     bool tree_built = false;           // a tree exists (freeze_tree keeps it)
     std::vector<qz::DBuf<int>> node_of; // per level: node of each particle or -1
     qz::DBuf<int> amr_tmp, amr_tmp2;   // scratch (labels, scans, compaction)
-    qz::DBuf<int> zone_box;            // per zone: min x,y,z, max x,y,z
-    qz::DBuf<int> zone_cells;          // per zone: cells
-    qz::DBuf<int> gather_idx;          // small gathers of scan values
+    qz::DBuf<int> zone_box;            // a level's zone record (k_zone_roots)
     qz::DBuf<double> seg_mass;         // per deposit segment: mass
     // on-chip conjugate gradient: exchanged words (halo values, partial sums) and the
     // next launch's first tag, ghost lists, brick scratch; cgr_ghosts (tests) caps the
