@@ -951,12 +951,45 @@ int qz_step(qz_sim *s, double dt, int nsteps)
     return check_flags(s);
 }
 
+} // extern "C"
+
+// Arrays moved between page-locked host memory and the device by loads and stores, one
+// launch for all of them: what nineteen short transfers cost is queueing and starting each.
+struct CopyList {
+    const double *src[10];
+    double *dst[10];
+};
+
+__global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L)
+{
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        L.dst[blockIdx.y][i] = L.src[blockIdx.y][i];
+}
+
+// Up to this many particles.  A head-only step from page-locked arrays, 32^3 head, us, with
+// transfers and with loads: 2,000 particles 214 and 164, 10,000 245 and 205, 20,000 271 and
+// 237, 40,000 326 and 300, 65,536 386 and 378, 100,000 468 and 483, a million 2,846 and
+// 3,267.  The line lies below the crossing because transfers of the positions back overlap
+// the forces, which a refined step of some 50,000 particles gains from.
+constexpr long HOST_LOADS_MAX = 32768;
+
+static int copy_arrays(qz_sim *s, long n, int arrays, const CopyList &L)
+{
+    launch(s, QZ_PROF_OTHER, 16.0 * n * arrays, k_copy_arrays, dim3(blocks_for(n, 256), arrays),
+           dim3(256), n, L);
+    return check_cuda(cudaGetLastError(), "host arrays") ? QZ_SUCCESS : QZ_FAILURE;
+}
+
+extern "C" {
+
 // One step on host-resident state.  Page-locked arrays (every one of the ten):
 // x..vz and ax..az go in on the simulation's stream, the masses on a second
 // stream beside them and the kick-drift (the deposit is the first stage that
 // reads them), and the drifted positions come back on the second stream
 // while the forces are computed; velocities and accelerations come back after
-// the kick.  Pageable arrays: the staged copies of qz_set_particles /
+// the kick.  Up to HOST_LOADS_MAX particles one kernel moves the arrays in and one
+// moves them out instead.  Pageable arrays: the staged copies of qz_set_particles /
 // qz_get_particles around qz_step.  The arithmetic is qz_step's either way.
 int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *vx, double *vy,
                  double *vz, const double *m, double *ax, double *ay, double *az)
@@ -968,13 +1001,16 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
     }
     const long n = s->n;
     const void *arrays[10] = {x, y, z, vx, vy, vz, m, ax, ay, az};
-    bool pinned = true;
-    for (const void *p : arrays)
+    bool pinned = true, loads = n <= HOST_LOADS_MAX;
+    double *mapped[10]; // the arrays' device addresses
+    for (int q = 0; q < 10; q++)
     {
-        cudaPointerAttributes at;
-        pinned = pinned && cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+        cudaPointerAttributes at{};
+        pinned = pinned && cudaPointerGetAttributes(&at, arrays[q]) == cudaSuccess &&
                  at.type == cudaMemoryTypeHost;
         cudaGetLastError();
+        mapped[q] = (double *)at.devicePointer;
+        loads = loads && mapped[q] && (uintptr_t)mapped[q] % sizeof(double) == 0;
     }
     // outflow boundaries remove particles in the kick-drift: the plain sequence
     if (!pinned || s->cfg.bdry == 2 || n == 0)
@@ -983,6 +1019,34 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
                 qz_get_particles(s, x, y, z, vx, vy, vz, ax, ay, az))
                    ? QZ_FAILURE
                    : QZ_SUCCESS;
+    if (loads)
+    {
+        // x..vz, m and ax..az in one launch, x..vz and ax..az back in another
+        const CopyList in = {{mapped[0], mapped[1], mapped[2], mapped[3], mapped[4], mapped[5],
+                              mapped[6], mapped[7], mapped[8], mapped[9]},
+                             {s->x, s->y, s->z, s->vx, s->vy, s->vz, s->m, s->ax, s->ay, s->az}};
+        const CopyList out = {{s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az},
+                              {mapped[0], mapped[1], mapped[2], mapped[3], mapped[4], mapped[5],
+                               mapped[7], mapped[8], mapped[9]}};
+        s->head_mass = s->cfg.total_mass;
+        s->ofl_removed = 0;
+        s->forces_ready = true;
+        StepPending sp;
+        const bool ok = !copy_arrays(s, n, 10, in) && !kick_drift(s, dt) &&
+                        !tree_density_potential(s, sp) && !qz_grid_acceleration(s) &&
+                        !gather_kick(s, dt) && !copy_arrays(s, n, 9, out);
+        if (step_finish(s, sp) || !ok)
+        {
+            if (!ok)
+                copy_arrays(s, n, 3, out); // the drifted positions, as by copies
+            cudaStreamSynchronize(s->stream);
+            return QZ_FAILURE;
+        }
+        s->stats.steps++;
+        s->stats.last_dt = dt;
+        s->stats.sim_time += dt;
+        return check_flags(s);
+    }
     if (!s->xfer &&
         (!check_cuda(cudaStreamCreateWithFlags(&s->xfer, cudaStreamNonBlocking), "copy stream") ||
          !check_cuda(cudaEventCreateWithFlags(&s->ev_mass, cudaEventDisableTiming), "event") ||
