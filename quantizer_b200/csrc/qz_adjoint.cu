@@ -208,56 +208,48 @@ __global__ void __launch_bounds__(ADJ_SEG_LONG_THREADS)
 }
 
 // Each grid point sums the corner contributions of its (up to) 8 adjacent
-// occupied cells in a fixed order, three components.
-__global__ void k_adj_point_gather(long D, const int *__restrict__ cell_seg,
+// occupied cells in a fixed order, three components; a plane of points a row of blocks
+// (inv: div_magic(D)), the eight cells' loads in flight together.
+__global__ void k_adj_point_gather(int D, unsigned inv, const int *__restrict__ cell_seg,
                                    const double *__restrict__ cs, double *__restrict__ Abx,
                                    double *__restrict__ Aby, double *__restrict__ Abz)
 {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= D * D * D)
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (unsigned)(D * D))
         return;
-    const long B = D - 1;
-    int gx = (int)(t % D), gy = (int)((t / D) % D), gz = (int)(t / (D * D));
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int c = 0; c < 2; c++)
+    const int B = D - 1, gz = (int)blockIdx.y, gy = (int)__umulhi(q, inv), gx = (int)q - gy * D;
+    int sg[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++)
     {
-        int cz = gz - 1 + c;
-        if (cz < 0 || cz >= B)
-            continue;
-        for (int b = 0; b < 2; b++)
-        {
-            int cy = gy - 1 + b;
-            if (cy < 0 || cy >= B)
-                continue;
-            for (int a = 0; a < 2; a++)
-            {
-                int cx = gx - 1 + a;
-                if (cx < 0 || cx >= B)
-                    continue;
-                int sg = cell_seg[cx + cy * B + (long)cz * B * B];
-                if (sg >= 0)
-                {
-                    const int corner = (1 - a) + 2 * (1 - b) + 4 * (1 - c);
-                    a0 += cs[(long)sg * 24 + corner];
-                    a1 += cs[(long)sg * 24 + 8 + corner];
-                    a2 += cs[(long)sg * 24 + 16 + corner];
-                }
-            }
-        }
+        const int cx = gx - 1 + (o & 1), cy = gy - 1 + ((o >> 1) & 1), cz = gz - 1 + (o >> 2);
+        const bool in = cx >= 0 && cx < B && cy >= 0 && cy < B && cz >= 0 && cz < B;
+        sg[o] = in ? cell_seg[cx + (cy + cz * B) * B] : -1;
     }
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+#pragma unroll
+    for (int o = 0; o < 8; o++)
+        if (sg[o] >= 0)
+        {
+            const double *c = cs + (long)sg[o] * 24 + (7 - o);
+            a0 += c[0];
+            a1 += c[8];
+            a2 += c[16];
+        }
+    const long t = (long)gz * D * D + q;
     Abx[t] = a0;
     Aby[t] = a1;
     Abz[t] = a2;
 }
 
 // ---- gradient transpose -------------------------------------------------------------------
-__device__ __forceinline__ bool adj_interior(long i, long j, long k, int hi)
+__device__ __forceinline__ bool adj_interior(int i, int j, int k, int hi)
 {
     return i >= 2 && i <= hi && j >= 2 && j <= hi && k >= 2 && k <= hi;
 }
 
 // -div of Abar taken over the interior points where the gradient is evaluated.
-__device__ __forceinline__ double adj_negdiv(long i, long j, long k, long D, int hi, double o2h,
+__device__ __forceinline__ double adj_negdiv(int i, int j, int k, long D, int hi, double o2h,
                                              const double *__restrict__ Abx,
                                              const double *__restrict__ Aby,
                                              const double *__restrict__ Abz)
@@ -280,22 +272,26 @@ __device__ __forceinline__ double adj_negdiv(long i, long j, long k, long D, int
     return v * o2h;
 }
 
-__global__ void k_adj_negdiv(int L, long D, double o2h, const double *__restrict__ Abx,
+// A plane of interior points a row of blocks (inv: div_magic(2^L - 1)).
+__global__ void k_adj_negdiv(int L, unsigned inv, long D, double o2h, const double *__restrict__ Abx,
                              const double *__restrict__ Aby, const double *__restrict__ Abz,
                              double *__restrict__ phib)
 {
     const int m = (1 << L) - 1;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)m * m * m)
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (unsigned)(m * m))
         return;
-    const long i = 2 + t % m, j = 2 + (t / m) % m, k = 2 + t / ((long)m * m);
+    const unsigned row = __umulhi(q, inv);
+    const int i = 2 + (int)(q - row * m), j = 2 + (int)row, k = 2 + (int)blockIdx.y;
     phib[i + j * D + k * D * D] = adj_negdiv(i, j, k, D, 1 << L, o2h, Abx, Aby, Abz);
 }
 
 // ---- total-mass term ----------------------------------------------------------------------
 // Per block: sum over the solve grid's boundary points b (coordinates in
 // 1..2^L+1, one of them 1 or 2^L+1) of
-// phi_b (phibar_b - (1/H^2) sum of lam at the 6 neighbours) + Abar_b . A_b.
+// phi_b (phibar_b - (1/H^2) sum of lam at the 6 neighbours) + Abar_b . A_b.  The
+// two z faces, then the rims of the planes between them (at 128^3 a walk over the whole
+// grid that skips the inside took 31 us, the boundary alone 11).
 __global__ void k_adj_shell(int L, long D, double o2h, double oh2, const double *__restrict__ pot,
                             const double *__restrict__ lam, const double *__restrict__ Abx,
                             const double *__restrict__ Aby, const double *__restrict__ Abz,
@@ -305,15 +301,34 @@ __global__ void k_adj_shell(int L, long D, double o2h, double oh2, const double 
 {
     __shared__ double sh[32];
     const int n = (1 << L) + 1, hi = 1 << L;
-    const long total = (long)n * n * n;
+    const int faces = 2 * n * n, rim = 4 * (n - 1), total = faces + (n - 2) * rim;
     const long D2 = D * D;
     double acc = 0.0;
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (long)gridDim.x * blockDim.x)
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
     {
-        const long i = 1 + t % n, j = 1 + (t / n) % n, k = 1 + t / ((long)n * n);
-        if (adj_interior(i, j, k, hi))
-            continue;
+        int i, j, k;
+        if (t < faces)
+        {
+            const int row = t / n;
+            i = 1 + t - row * n;
+            j = 1 + (row < n ? row : row - n);
+            k = row < n ? 1 : n;
+        }
+        else
+        {
+            const int plane = (t - faces) / rim, r = t - faces - plane * rim;
+            k = 2 + plane;
+            if (r < 2 * n)
+            {
+                i = 1 + (r < n ? r : r - n);
+                j = r < n ? 1 : n;
+            }
+            else
+            {
+                i = r & 1 ? n : 1;
+                j = 2 + ((r - 2 * n) >> 1);
+            }
+        }
         const long g = i + j * D + k * D2;
         const double nb = lam[g + 1] + lam[g - 1] + lam[g + D] + lam[g - D] + lam[g + D2] +
                           lam[g - D2];
@@ -655,7 +670,7 @@ __global__ void k_adj_lvl_negdiv(long total, int nn, const AmrNode *__restrict__
 
 // per node: sum of rhs^2 over its interior list, in a fixed order: block (node, j) adds
 // the j-th of ADJ_NORM_PARTS slices, the second kernel the slices (one block a node
-// took 290 us for 100,000 points, mostly waiting for its loads; now 8)
+// took 290 us for 100,000 points, mostly waiting for its loads; both kernels now 11)
 constexpr int ADJ_NORM_PARTS = 64;
 
 __global__ void k_adj_node_norm(const AmrNode *__restrict__ nodes, const int *__restrict__ intr,
@@ -747,33 +762,66 @@ __global__ void k_adj_bdry_keys(int nlist, const int *__restrict__ list, const i
     val[t] = (int)t;
 }
 
-__global__ void k_adj_bdry_sum(long m, const unsigned *__restrict__ key, const int *__restrict__ val,
-                               const int *__restrict__ list, const int *__restrict__ lnode,
-                               const AmrNode *__restrict__ nodes, const double *__restrict__ phib,
-                               const double *__restrict__ lam, const double *__restrict__ A0,
-                               const double *__restrict__ A1, const double *__restrict__ A2,
-                               double *__restrict__ pA0, double *__restrict__ pA1,
-                               double *__restrict__ pA2, double *__restrict__ pphic)
+// Sum of every run of equal keys, in the order of the sort.  All entries' values are
+// worked out side by side, a block's and the BS_HALO after them (a parent point has up to
+// 64 entries of one node; what is left of a longer run is worked out by its first thread),
+// and the run's first thread adds them from shared memory.  A level of 262,144 particles
+// on a 128^3 head: 12 us, 52 with that thread working through its run's chains of loads.
+constexpr int BS_THREADS = 256, BS_HALO = 64;
+
+__global__ void __launch_bounds__(BS_THREADS)
+    k_adj_bdry_sum(long m, const unsigned *__restrict__ key, const int *__restrict__ val,
+                   const int *__restrict__ list, const int *__restrict__ lnode,
+                   const AmrNode *__restrict__ nodes, const double *__restrict__ phib,
+                   const double *__restrict__ lam, const double *__restrict__ A0,
+                   const double *__restrict__ A1, const double *__restrict__ A2,
+                   double *__restrict__ pA0, double *__restrict__ pA1, double *__restrict__ pA2,
+                   double *__restrict__ pphic)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || (i > 0 && key[i - 1] == key[i]))
-        return;
-    const unsigned q = key[i];
-    double sf = 0.0, s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (long j = i; j < m && key[j] == q; j++)
-    {
+    __shared__ double sv[4][BS_THREADS + BS_HALO];
+    __shared__ unsigned sk[BS_THREADS + BS_HALO];
+    const long i0 = (long)blockIdx.x * BS_THREADS;
+    auto entry = [&](long j, double (&v)[4]) {
         const int e = val[j] >> 3;
         const long g = list[e];
-        const AmrNode N = nodes[lnode[e]];
-        sf += 0.125 * adj_phit(N, g, phib, lam);
-        s0 += 0.125 * A0[g];
-        s1 += 0.125 * A1[g];
-        s2 += 0.125 * A2[g];
+        v[0] = 0.125 * adj_phit(nodes[lnode[e]], g, phib, lam);
+        v[1] = 0.125 * A0[g];
+        v[2] = 0.125 * A1[g];
+        v[3] = 0.125 * A2[g];
+    };
+    for (int q = threadIdx.x; q < BS_THREADS + BS_HALO && i0 + q < m; q += BS_THREADS)
+    {
+        double v[4];
+        entry(i0 + q, v);
+        sk[q] = key[i0 + q];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            sv[c][q] = v[c];
     }
-    pphic[q] += sf;
-    pA0[q] += s0;
-    pA1[q] += s1;
-    pA2[q] += s2;
+    __syncthreads();
+    const long i = i0 + threadIdx.x;
+    if (i >= m || (i > 0 && key[i - 1] == key[i]))
+        return;
+    const unsigned k = sk[threadIdx.x];
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int q = threadIdx.x;
+    for (; q < BS_THREADS + BS_HALO && i0 + q < m && sk[q] == k; q++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            s[c] += sv[c][q];
+    if (q == BS_THREADS + BS_HALO)
+        for (long j = i0 + q; j < m && key[j] == k; j++)
+        {
+            double v[4];
+            entry(j, v);
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                s[c] += v[c];
+        }
+    pphic[k] += s[0];
+    pA0[k] += s[1];
+    pA1[k] += s[2];
+    pA2[k] += s[3];
 }
 
 // simulation-boundary points (analytic, linear in M): per block partial sums of
@@ -1137,8 +1185,8 @@ static int force_vjp(qz_sim *s, const double *x, const double *y, const double *
     launch(s, QZ_PROF_DEPOSIT, 0.0, k_adj_seg_long, dim3(2 * sms), dim3(ADJ_SEG_LONG_THREADS), L, perm,
            s->seg_start, s->flags, s->long_seg, x, y, z, abh, abh + n, abh + 2 * n, A.cs.p);
     double *Abx = A.Ab.p, *Aby = A.Ab.p + s->gpts, *Abz = A.Ab.p + 2 * s->gpts;
-    launch(s, QZ_PROF_DEPOSIT, 24.0 * s->gpts, k_adj_point_gather, dim3(blocks_for(s->gpts, 256)),
-           dim3(256), D, s->cell_seg, A.cs.p, Abx, Aby, Abz);
+    launch(s, QZ_PROF_DEPOSIT, 24.0 * s->gpts, k_adj_point_gather, dim3(blocks_for(D * D, 256), (unsigned)D),
+           dim3(256), (int)D, div_magic((unsigned)D), s->cell_seg, A.cs.p, Abx, Aby, Abz);
     if (amr)
     {
         // the finest-level gathers' transposes, then the levels from the finest down
@@ -1243,7 +1291,7 @@ static int force_vjp(qz_sim *s, const double *x, const double *y, const double *
                 if (radix_sort_pairs(s, m8, bits, &bk, &bv))
                     return QZ_FAILURE;
                 launch(s, QZ_PROF_OTHER, 160.0 * Lv.bdry_total, k_adj_bdry_sum,
-                       dim3(blocks_for(m8, 256)), dim3(256), m8, bk, bv, Lv.bdry.p,
+                       dim3(blocks_for(m8, BS_THREADS)), dim3(BS_THREADS), m8, bk, bv, Lv.bdry.p,
                        Lv.bdry_node.p, Lv.nodes.p, A.lphib[l].p, A.llam[l].p, A0, A1, A2, pA0,
                        pA1, pA2, pphic);
             }
@@ -1264,8 +1312,8 @@ static int force_vjp(qz_sim *s, const double *x, const double *y, const double *
         }
     }
     const long m = (1L << L) - 1;
-    launch(s, QZ_PROF_GRADIENT, 32.0 * m * m * m, k_adj_negdiv, dim3(blocks_for(m * m * m, 256)),
-           dim3(256), L, D, o2h, Abx, Aby, Abz, A.phib.p);
+    launch(s, QZ_PROF_GRADIENT, 32.0 * m * m * m, k_adj_negdiv, dim3(blocks_for(m * m, 256), (unsigned)m),
+           dim3(256), L, div_magic((unsigned)m), D, o2h, Abx, Aby, Abz, A.phib.p);
     if (amr)
         launch(s, QZ_PROF_GRADIENT, 16.0 * m * m * m, k_adj_add_interior,
                dim3(blocks_for(m * m * m, 256)), dim3(256), L, D, A.phic0.p, A.phib.p);

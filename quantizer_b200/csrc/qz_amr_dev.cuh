@@ -38,12 +38,13 @@ __device__ __forceinline__ long grid_index(const AmrNode &N, int gx, int gy, int
 
 __device__ __forceinline__ void grid_coords(const AmrNode &N, long g, int *gx, int *gy, int *gz)
 {
-    long l = g - N.grid_off;
-    const long sx = N.rd[0] + 1, sxy = sx * (N.rd[1] + 1);
-    *gz = (int)(l / sxy);
-    l -= (long)(*gz) * sxy;
-    *gy = (int)(l / sx);
-    *gx = (int)(l - (long)(*gy) * sx);
+    // 32 bits hold a place in a node's grid, as the point lists do, and divide in a fraction
+    // of the instructions (k_lvl_point_gather on 4.6M points: 77 to 72 us)
+    const unsigned l = (unsigned)(g - N.grid_off), sx = N.rd[0] + 1, sy = N.rd[1] + 1;
+    const unsigned row = l / sx, plane = row / sy;
+    *gz = (int)plane;
+    *gy = (int)(row - plane * sy);
+    *gx = (int)(l - row * sx);
 }
 
 // Parent-interpolated start (potential_branches.c:204-331): 0.125 times the sum

@@ -249,7 +249,7 @@ __device__ __forceinline__ void head_cic_add(int i, double scale, double coeff,
 
 // The corner sums of every occupied cell of at most SEG_LONG particles; longer cells are
 // listed for k_seg_long.  262,144 particles on a 128^3 head: 30.5 us with a warp a cell
-// and a full xor tree a sum, 13 in groups of lanes with shared exchanges.
+// and a full xor tree a sum, 21 in groups of lanes with shared exchanges.
 __global__ void k_seg_reduce(int L, double coeff, const int *__restrict__ perm,
                              const int *__restrict__ seg_start, int *__restrict__ flags,
                              int *__restrict__ long_list, const double *__restrict__ x,

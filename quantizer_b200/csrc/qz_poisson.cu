@@ -2269,14 +2269,13 @@ __global__ void k_resid_norm_partial(int L, long D, const double *__restrict__ l
                                      double *__restrict__ partial)
 {
     __shared__ double sh[32];
-    const int m = (1 << L) - 1;
-    const long total = (long)m * m * m;
+    const unsigned m = (1u << L) - 1, total = m * m * m;
     const long D2 = D * D;
     double rr = 0.0, ff = 0.0;
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (long)gridDim.x * blockDim.x)
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
     {
-        const long i = 2 + t % m, j = 2 + (t / m) % m, k = 2 + t / ((long)m * m);
+        const unsigned row = t / m, plane = row / m;
+        const long i = 2 + (t - row * m), j = 2 + (row - plane * m), k = 2 + plane;
         const long g = i + j * D + k * D2;
         const double r = f[g] + oh2 * (6.0 * lam[g] - lam[g + 1] - lam[g - 1] - lam[g + D] -
                                        lam[g - D] - lam[g + D2] - lam[g - D2]);

@@ -239,7 +239,7 @@ __global__ void k_rs_hist(const unsigned *__restrict__ keys, long n, int passes,
 // consecutive stores.  A pass is a chain of trips (tile number, keys, look-back,
 // stores) rather than bytes: with 2048-key tiles, keys loaded twice one iteration at a
 // time, one predecessor a trip and scattered stores it took 14 us at 10,000 keys and
-// 31 at 1M; now 7 and 17.
+// 31 at 1M; now 8 and 24.
 __global__ void __launch_bounds__(RS_WARPS * 32)
     k_rs_onesweep(const unsigned *__restrict__ kin, const int *__restrict__ vin,
                   unsigned *__restrict__ kout, int *__restrict__ vout, long n, int shift,
