@@ -98,13 +98,20 @@ typedef struct qz_config {
     /* adjoint Poisson solves (qz_force_vjp, qz_adjoint_final_loss): multigrid
      * cycles until |r| <= adjoint_tol |rhs| (2-norms over the head interior) */
     double adjoint_tol;
-    /* refinement-node conjugate gradient: 0 the reference's two reductions per
-     * iteration, 1 one reduction per iteration (Chronopoulos-Gear arrangement:
+    /* refinement-node conjugate gradient: 0 (default) the vectors on chip, in
+     * registers and shared memory, one exchange an iteration (Chronopoulos-Gear
+     * arrangement; a level whose nodes do not fit, and a node with points on its
+     * grid's faces, runs the reference's two reductions per iteration from
+     * device memory), 1 from device memory with one reduction per iteration (Chronopoulos-Gear arrangement:
      * the same iterates in exact arithmetic, half the waits), 2 one reduction
      * per iteration in the pipelined arrangement (Ghysels-Vanroose: w = A r
      * by recurrence, one stencil and 12 loads a point) */
     int cg_variant;
-    /* persistent multigrid cycles: finest-level points of one colour per thread,
+    /* A head solve by red-black Gauss-Seidel V-cycles of at least 100 allowed
+     * iterations, with no recorded or replayed schedule, starts with a direct
+     * solution by sine transforms; cycles run only where the convergence test
+     * does not hold for it.
+     * persistent multigrid cycles: finest-level points of one colour per thread,
      * which sets the launch's block count (at most two blocks per SM); results
      * do not depend on it (qz_ensemble_autotune picks it for ensembles) */
     int mg_points_per_thread;
@@ -134,15 +141,16 @@ typedef struct qz_config {
      * does (0, default): fewer iterations, the same convergence test, results
      * that differ from the reference's by the solve tolerance */
     int node_warm;
-    /* refinement steps whose head solve is one persistent launch: 1 (default)
-     * runs that launch on a second stream of higher priority while the tree
+    /* refinement steps whose head solve is queued without a host wait (the direct
+     * solve and the persistent cycles behind it): 1 (default) runs it on a second stream of higher priority while the tree
      * construction and the level deposits, which read only the particles, run
      * on the simulation's stream; the level solves start when both are done.
      * 0 runs the stages one after another in main.c's order.  Results are the
      * same bit for bit either way. */
     int tree_overlap;
     /* refinement-node conjugate gradient: fewest interior points in a chunk
-     * (one 512-thread block works a chunk; chunks never cross nodes).  0
+     * (one block works a chunk; chunks never cross nodes; the on-chip form counts
+     * rows of four points).  0
      * (default): a level's points are cut into about 148 chunks, one a SM,
      * which suits one simulation on the GPU.  Many simulations side by side
      * (qz_ensemble_step) want larger chunks, e.g. 2048, so that a small
@@ -161,7 +169,8 @@ typedef struct qz_config {
 
 typedef struct qz_stats {
     long long vcycles_total;   /* V-cycles (FP64 or FP32 inner) since creation */
-    int last_vcycles;          /* V-cycles of the last potential solve */
+    int last_vcycles;          /* V-cycles of the last potential solve; 0 when the direct
+                                  solve (sine transforms) passed the convergence test */
     int last_converged;        /* 1 if the last solve met both thresholds */
     long long kernel_launches; /* kernels this library launched since creation */
     long long steps;           /* completed qz_step steps */

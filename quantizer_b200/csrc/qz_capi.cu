@@ -783,10 +783,12 @@ namespace qz {
 // built and the levels deposited on the simulation's stream, with the host
 // waits of the tree construction overlapping the solve; the level solves wait
 // for both.  Every kernel computes what it computes in the sequential order.
-// Measured on the 1M-particle sphere (128^3 head, three levels), ms a step:
-// sequential 10.54-10.59; overlapped with 4 points a thread (two blocks on
+// The launch's cycles take this many points a thread, measured on the 1M-particle
+// sphere (128^3 head, three levels) with ten cycles a step and nothing before them,
+// ms a step: sequential 10.54-10.59; overlapped with 4 points a thread (two blocks on
 // every SM: the tree kernels wait for the solve) 10.61, 8 points 9.66-9.80,
-// 10 points 9.57, 12 points 9.53, 16 points 9.95.
+// 10 points 9.57, 12 points 9.53, 16 points 9.95.  Where the direct solution passes, no
+// cycle runs and 0.14 ms of transforms are what overlaps.
 constexpr int OVERLAP_PPT = 12;
 
 // Outcomes a step reads at its end: the head launch (when it was queued) and the queued level solves.

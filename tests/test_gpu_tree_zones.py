@@ -1,8 +1,9 @@
 """GPU: the refinement tree and the levels' densities against a plain numpy construction,
 on zone shapes at which the union-find, the ordered selections and the segment sums have
 their edges: one cell, long chains that turn back (their parents lead far), staircases in
-both directions, many small zones, one large one, zones on the simulation's boundary, and
-particle numbers at the edges of the sort's tiles and of the cells' segments.
+both directions, 1,728 small zones (of more cells than the sort has room for particles), one
+large one, zones on the simulation's boundary, and particle numbers at the
+edges of the sort's tiles and of the cells' segments.
 
 The construction: a cell with ref_ptcl particles or more and its neighbours in the node
 are refined; zones are 6-connected (scipy.ndimage.label); cells, nodes and point lists in
@@ -18,7 +19,7 @@ from quantizer_b200 import core
 
 pytestmark = pytest.mark.gpu
 
-LMIN, REF = 5, 3
+REF = 3
 
 
 def _snake():
@@ -35,6 +36,9 @@ def _seeds(name):
     rng = np.random.default_rng(11)
     if name == "one":
         return [(9, 14, 20)]
+    if name == "many":  # 1,728 zones on a head of 64
+        return [(4 * i + 2, 4 * j + 2, 4 * k + 2) for k in range(12) for j in range(12)
+                for i in range(12)]
     if name == "corners":
         return [(0, 0, 0), (31, 31, 31), (0, 31, 16)]
     if name == "snake":
@@ -49,16 +53,16 @@ def _seeds(name):
     return [tuple(c) for c in rng.integers(1, 31, (420, 3))]  # "dense": one ragged zone
 
 
-def _particles(name, extra):
+def _particles(name, extra, cells):
     """REF particles in every seed cell, some of them close enough together to refine
     a level further; `extra` more in one cell (a long segment)."""
     rng = np.random.default_rng(5)
     pos = []
     for k, c in enumerate(dict.fromkeys(_seeds(name))):
         w = 0.5 if k % 3 == 0 else 1.0
-        pos.append((np.array(c) + w * rng.uniform(0.02, 0.98, (REF, 3))) / 32)
+        pos.append((np.array(c) + w * rng.uniform(0.02, 0.98, (REF, 3))) / cells)
     c = np.array(_seeds(name)[0])
-    pos.append((c + rng.uniform(0.02, 0.98, (extra, 3))) / 32)
+    pos.append((c + rng.uniform(0.02, 0.98, (extra, 3))) / cells)
     pos = np.concatenate(pos)
     return pos[rng.permutation(len(pos))]
 
@@ -101,34 +105,35 @@ def _zones(cells, pos, lv):
 
 
 CASES = [("one", 0), ("one", 253), ("one", 254), ("corners", 300), ("snake", 2), ("stairs", 2500),
-         ("ball", 0), ("sparse", 3916), ("dense", 70)]
+         ("ball", 0), ("sparse", 3916), ("dense", 70), ("many", 0)]
 
 
 @pytest.mark.parametrize("name,extra", CASES)
 def test_tree_and_density(name, extra):
-    pos = _particles(name, extra)
+    lmin = 6 if name == "many" else 5
+    pos = _particles(name, extra, 1 << lmin)
     n = len(pos)
     rng = np.random.default_rng(1)
     ic = {k: np.ascontiguousarray(pos[:, q]) for q, k in enumerate("xyz")}
     ic.update({k: np.zeros(n) for k in ("vx", "vy", "vz")})
     ic["m"] = rng.uniform(0.5, 1.5, n) / n
     seen = 0
-    with core.Simulation(ic, LMIN, lmax=LMIN + 2, ref_ptcl=REF) as sim:
+    with core.Simulation(ic, lmin, lmax=lmin + 2, ref_ptcl=REF) as sim:
         sim.tree_adaptation()
         sim.grid_density()
-        g = np.arange(32)
+        g = np.arange(1 << lmin)
         z, y, x = np.meshgrid(g, g, g, indexing="ij")
         nodes = [(np.stack([x.ravel(), y.ravel(), z.ravel()], 1), np.arange(n))]
         for level in (1, 2):
-            lv, children = LMIN + level, []
+            lv, children = lmin + level, []
             for parent, (cells, ptcl) in enumerate(nodes):
                 for zone in _zones(cells, pos[ptcl], lv - 1):
                     zc = cells[zone]
                     sub = np.array([(s & 1, s >> 1 & 1, s >> 2) for s in range(8)])
                     mine = (2 * zc[:, None, :] + sub[None]).reshape(-1, 3)
-                    keys = set(map(tuple, zc))
                     pc = np.floor(pos[ptcl] * (1 << (lv - 1))).astype(int)
-                    here = np.array([tuple(c) in keys for c in pc], dtype=bool)
+                    place = 1 << 10 * np.arange(3)
+                    here = np.isin(pc @ place, zc @ place)
                     children.append((mine, ptcl[here], parent))
             assert (sim.num_nodes(level) if level < sim.levels() else 0) == len(children)
             for q, (cells, ptcl, parent) in enumerate(children):
