@@ -554,6 +554,8 @@ int qz_create(const qz_config *cfg, long n_capacity, qz_sim **out)
         if (ok)
             s->fine_alt = head_view(s, s->fine_alt_buf);
     }
+    if (ok && direct_allowed(s))
+        ok = direct_tables(s);
     if (ok)
         ok = head_initial(s) == QZ_SUCCESS;
     if (ok && cfg->lmax > cfg->lmin)

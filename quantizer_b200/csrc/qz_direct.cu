@@ -372,10 +372,10 @@ __global__ void __launch_bounds__(DC_THREADS)
 
 // ---- host ---------------------------------------------------------------------------------
 // Twiddles exp(-2 pi i q / 2N), q < 2N, then the eigenvalues 2 cos(pi k / N) - 2, k < N.
-static bool direct_tables(qz_sim *s)
+// Made with the simulation and waited for there: the passes run on streams that no copy on
+// the default stream precedes, and a copy from pageable memory returns before it has arrived.
+bool direct_tables(qz_sim *s)
 {
-    if (s->direct_tab)
-        return true;
     const int N = 1 << s->L;
     std::vector<double> h(4 * N + N);
     const long double pi = 3.14159265358979323846264338327950288L;
@@ -392,14 +392,10 @@ static bool direct_tables(qz_sim *s)
     double *p = nullptr;
     if (!check_cuda(cudaMalloc((void **)&p, h.size() * sizeof(double)), "sine tables"))
         return false;
-    if (!check_cuda(cudaMemcpy(p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice),
-                    "sine tables"))
-    {
-        cudaFree(p);
-        return false;
-    }
     s->direct_tab = p;
-    return true;
+    return check_cuda(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(double),
+                                      cudaMemcpyHostToDevice, s->stream), "sine tables") &&
+           check_cuda(cudaStreamSynchronize(s->stream), "sine tables");
 }
 
 template <int LG>
@@ -431,8 +427,6 @@ static void direct_passes(qz_sim *s, Grid<double> phi, Grid<double> rho, const i
 // transforms' work space.
 static int direct_correct_unless(qz_sim *s, double *phi, double *rho, const int *done)
 {
-    if (!direct_tables(s))
-        return QZ_FAILURE;
     const Grid<double> p = head_view(s, phi), r = head_view(s, rho);
     switch (s->L)
     {

@@ -746,7 +746,9 @@ int kick_drift(qz_sim *s, double dt);
 int kick(qz_sim *s, double dt);
 
 int potential_head(qz_sim *s);
-int direct_correct(qz_sim *s, double *phi, double *rho); // qz_direct.cu
+bool direct_allowed(const qz_sim *s); // by the configuration alone
+bool direct_tables(qz_sim *s);        // qz_direct.cu
+int direct_correct(qz_sim *s, double *phi, double *rho);
 int direct_head(qz_sim *s);
 int amr_init(qz_sim *s);
 void amr_free(qz_sim *s);

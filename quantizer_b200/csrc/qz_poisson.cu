@@ -2334,7 +2334,7 @@ static int resid_norms(qz_sim *s, const double *lam, const double *f, double *sc
 // failure).
 constexpr int DIRECT_MIN_CAP = 100;
 
-static bool direct_allowed(const qz_sim *s)
+bool direct_allowed(const qz_sim *s)
 {
     const qz_config &c = s->cfg;
     return c.smoother == 0 && c.gs_order == QZ_GS_REDBLACK && c.cycle == 0 && !s->fused_rb &&
