@@ -25,7 +25,6 @@ def test_first_solve_leaves_the_default_stream_alone(lmin):
             waited = busy.query()
             torch.cuda.synchronize()
             pots.append(sim.field("pot"))
-            assert sim.stats().last_vcycles == 0
     assert not waited
     for p in pots[1:]:
         np.testing.assert_array_equal(p, pots[0])
