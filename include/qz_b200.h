@@ -283,7 +283,12 @@ QZ_API int qz_amr_node_field(qz_sim *sim, int level, int node, int which, double
 
 /* Step 0 force computation (main.c:296-338) and whole leapfrog steps
  * (main.c:375-481).  dt > 0: that fixed step; dt <= 0: each step takes the
- * CFL step of qz_timestep from the current state, as main.c:375 does. */
+ * CFL step of qz_timestep from the current state, as main.c:375 does.
+ * A step whose head solve fails ends there: drifted positions, the velocities of
+ * the first kick, no accelerations (qz_step_host: the caller's velocities and
+ * accelerations as they were).  In a refinement step whose level solves are queued
+ * (tree_overlap) the forces and the second kick are queued behind them, so one that
+ * fails leaves the velocities and accelerations of the potentials reached. */
 QZ_API int qz_init_forces(qz_sim *sim);
 QZ_API int qz_step(qz_sim *sim, double dt, int nsteps);
 

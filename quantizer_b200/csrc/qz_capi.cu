@@ -441,6 +441,8 @@ int qz_destroy(qz_sim *s)
         cudaEventDestroy(s->ev_fork);
     if (s->ev_head)
         cudaEventDestroy(s->ev_head);
+    if (s->ev_outcome)
+        cudaEventDestroy(s->ev_outcome);
     if (s->stream)
         cudaStreamDestroy(s->stream);
     delete s;
@@ -535,7 +537,8 @@ int qz_create(const qz_config *cfg, long n_capacity, qz_sim **out)
     s->red_blocks = 296;
     ok = ok && dmalloc(&s->red, s->red_blocks + 8, "red") && dmalloc(&s->flags, F_COUNT + F_OUTST, "flags");
     s->outst = s->flags + F_COUNT;
-    ok = ok && check_cuda(cudaMallocHost((void **)&s->h_flags, (F_COUNT + F_OUTST) * sizeof(int)), "pinned");
+    ok = ok && check_cuda(cudaMallocHost((void **)&s->h_flags, (F_COUNT + F_OUTST) * sizeof(int)), "pinned") &&
+         check_cuda(cudaEventCreateWithFlags(&s->ev_outcome, cudaEventDisableTiming), "event");
     ok = ok && dmalloc(&s->gbar, 4, "grid barrier");
     ok = ok && check_cuda(cudaMallocHost((void **)&s->h_ts, 34 * sizeof(unsigned long long)),
                           "pinned time step") &&
@@ -664,17 +667,21 @@ int qz_set_head_field(qz_sim *s, int which, const double *in)
 
 int qz_initial_potential_head(qz_sim *s) { return s ? head_initial(s) : QZ_FAILURE; }
 
+static bool zero_accelerations(qz_sim *s)
+{
+    const size_t b = (size_t)(s->n > 0 ? s->n : 1) * sizeof(double);
+    return check_cuda(cudaMemsetAsync(s->ax, 0, b, s->stream), "reset") &&
+           check_cuda(cudaMemsetAsync(s->ay, 0, b, s->stream), "reset") &&
+           check_cuda(cudaMemsetAsync(s->az, 0, b, s->stream), "reset");
+}
+
 // reset.c:29-64: particle accelerations and head density to zero.
 int qz_reset(qz_sim *s)
 {
-    if (!s)
-        return QZ_FAILURE;
-    size_t b = (size_t)(s->n > 0 ? s->n : 1) * sizeof(double);
-    bool ok = check_cuda(cudaMemsetAsync(s->ax, 0, b, s->stream), "reset") &&
-              check_cuda(cudaMemsetAsync(s->ay, 0, b, s->stream), "reset") &&
-              check_cuda(cudaMemsetAsync(s->az, 0, b, s->stream), "reset") &&
-              check_cuda(cudaMemsetAsync(s->d, 0, s->gpts * sizeof(double), s->stream), "reset");
-    return ok ? QZ_SUCCESS : QZ_FAILURE;
+    return s && zero_accelerations(s) &&
+                   check_cuda(cudaMemsetAsync(s->d, 0, s->gpts * sizeof(double), s->stream), "reset")
+               ? QZ_SUCCESS
+               : QZ_FAILURE;
 }
 
 static bool amr_on(const qz_sim *s) { return s->cfg.lmax > s->cfg.lmin; }
@@ -796,7 +803,6 @@ constexpr int OVERLAP_PPT = 12;
 // Outcomes a step reads at its end: the head launch (when it was queued) and the queued level solves.
 struct StepPending {
     bool head = false;
-    cudaStream_t head_stream = nullptr; // where the head launch is queued
     bool levels = false;
     std::vector<CgPending> pend;
 };
@@ -806,7 +812,7 @@ struct StepPending {
 static int step_finish(qz_sim *s, StepPending &sp)
 {
     int rc = QZ_SUCCESS;
-    if (sp.head && potential_head_finish(s, sp.head_stream))
+    if (sp.head && potential_head_finish(s))
         rc = QZ_FAILURE;
     if (rc == QZ_SUCCESS && sp.levels && amr_potential_collect(s, sp.pend))
         rc = QZ_FAILURE;
@@ -820,7 +826,6 @@ static int tree_density_potential(qz_sim *s, StepPending &sp)
     {
         // head only: the gradient, gather and kick are queued behind the head solve
         bool issued = false;
-        sp.head_stream = s->stream;
         if (deposit_head(s) || potential_head_issue(s, s->stream, &issued))
             return QZ_FAILURE;
         sp.head = issued;
@@ -862,7 +867,6 @@ static int tree_density_potential(qz_sim *s, StepPending &sp)
     // last level on the stream; the outcomes (head, then levels) are read at
     // the end of the step (step_finish)
     sp.head = true;
-    sp.head_stream = s->head_stream;
     if (ok && amr_potential_queues(s))
     {
         sp.levels = true;
@@ -871,17 +875,34 @@ static int tree_density_potential(qz_sim *s, StepPending &sp)
     }
     // the head launch is always waited for, whatever the other stages' outcome
     sp.head = false;
-    const bool head_ok = !potential_head_finish(s, s->head_stream);
+    const bool head_ok = !potential_head_finish(s);
     if (!ok || !head_ok)
         return QZ_FAILURE;
     return amr_potential(s);
 }
 
+// What a head-only step queues behind its head solve asks for the solve's outcome itself,
+// so that a step that fails ends with the drifted positions, the velocities of the first
+// kick and no accelerations, as if the host had read the outcome first.
+static HeadGate head_gate(const qz_sim *s, const StepPending &sp)
+{
+    return sp.head && !amr_on(s) ? HeadGate{s->outst, s->flags, s->cfg.max_iter} : HeadGate{};
+}
+
 // The gather and the kick of a step in one launch, from zero accelerations; with it a step
 // needs no reset (reset.c:29-64): the deposit writes every point of the head's density.
-static int gather_kick(qz_sim *s, double dt)
+static int gather_kick(qz_sim *s, double dt, const StepPending &sp)
 {
-    return amr_on(s) ? amr_gather(s, true, dt) : gather_head(s, true, dt);
+    return amr_on(s) ? amr_gather(s, true, dt) : gather_head(s, true, dt, head_gate(s, sp));
+}
+
+// Tree to kick; a step that fails before its gather has no accelerations either.
+static bool forces_kick(qz_sim *s, double dt, StepPending &sp)
+{
+    if (!tree_density_potential(s, sp) && !qz_grid_acceleration(s) && !gather_kick(s, dt, sp))
+        return true;
+    zero_accelerations(s);
+    return false;
 }
 
 // main.c:375-481 with a given dt: kick-drift, reset, tree, deposit, potential,
@@ -889,8 +910,7 @@ static int gather_kick(qz_sim *s, double dt)
 int step_core(qz_sim *s, double h)
 {
     StepPending sp;
-    const bool ok = !kick_drift(s, h) && !tree_density_potential(s, sp) &&
-                    !qz_grid_acceleration(s) && !gather_kick(s, h);
+    const bool ok = !kick_drift(s, h) && forces_kick(s, h, sp);
     if (step_finish(s, sp) || !ok)
         return QZ_FAILURE;
     s->stats.steps++;
@@ -964,10 +984,11 @@ struct CopyList {
     double *dst[10];
 };
 
-__global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L)
+// gate: past the first three arrays
+__global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L, HeadGate gate)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n)
+    if (i < n && (blockIdx.y < 3 || !head_failed(gate)))
         L.dst[blockIdx.y][i] = L.src[blockIdx.y][i];
 }
 
@@ -978,10 +999,10 @@ __global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L)
 // the forces, which a refined step of some 50,000 particles gains from.
 constexpr long HOST_LOADS_MAX = 32768;
 
-static int copy_arrays(qz_sim *s, long n, int arrays, const CopyList &L)
+static int copy_arrays(qz_sim *s, long n, int arrays, const CopyList &L, const HeadGate &gate = {})
 {
     launch(s, QZ_PROF_OTHER, 16.0 * n * arrays, k_copy_arrays, dim3(blocks_for(n, 256), arrays),
-           dim3(256), n, L);
+           dim3(256), n, L, gate);
     return check_cuda(cudaGetLastError(), "host arrays") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
@@ -1037,8 +1058,7 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
         s->forces_ready = true;
         StepPending sp;
         const bool ok = !copy_arrays(s, n, 10, in) && !kick_drift(s, dt) &&
-                        !tree_density_potential(s, sp) && !qz_grid_acceleration(s) &&
-                        !gather_kick(s, dt) && !copy_arrays(s, n, 9, out);
+                        forces_kick(s, dt, sp) && !copy_arrays(s, n, 9, out, head_gate(s, sp));
         if (step_finish(s, sp) || !ok)
         {
             if (!ok)
@@ -1078,10 +1098,12 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
         if (!check_cuda(cudaMemcpyAsync(hx[q], dx[q], b, cudaMemcpyDeviceToHost, s->xfer), "d2h"))
             return QZ_FAILURE;
     StepPending sp;
-    const bool ok = check_cuda(cudaStreamWaitEvent(s->stream, s->ev_mass, 0), "wait") &&
-                    !tree_density_potential(s, sp) && !qz_grid_acceleration(s) &&
-                    !gather_kick(s, dt);
-    // the copies back are queued before the step's outcomes are read
+    bool ok = check_cuda(cudaStreamWaitEvent(s->stream, s->ev_mass, 0), "wait") &&
+              forces_kick(s, dt, sp);
+    // the copies back are queued before the step's outcomes are read, but for the head-only
+    // step's, which is there while the gather is still to run
+    if (ok && !amr_on(s))
+        ok = !step_finish(s, sp);
     double *ho[6] = {vx, vy, vz, ax, ay, az};
     const double *dout[6] = {s->vx, s->vy, s->vz, s->ax, s->ay, s->az};
     bool copied = ok;

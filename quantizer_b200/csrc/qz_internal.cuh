@@ -138,6 +138,14 @@ __device__ __forceinline__ void apply_kick(const Kick &k, long i, double ax, dou
 }
 #endif
 
+// Outcome of a head solve that is queued before the kernels that take a gate: these leave
+// the particles as a step that ends at a failed solve does (potential_head_finish makes the
+// same test).  No outst: always open.
+struct HeadGate {
+    const int *outst, *flags;
+    int cap;
+};
+
 // Device-side flag words (int).
 enum Flag {
     F_RATIO_FAIL = 0, // ratio test |phi/phi_old - 1| > tol2 somewhere
@@ -151,6 +159,13 @@ enum Flag {
     F_OUTST = 4 // words of outst, after the flags
 };
 enum ErrorBits { E_PTCL_OUTSIDE = 1, E_SORT_RANGE = 2, E_BARRIER = 8, E_SCAN = 16 };
+
+#ifdef __CUDACC__
+__device__ __forceinline__ bool head_failed(const HeadGate &g)
+{
+    return g.outst && (g.outst[0] == g.cap || (g.flags[F_ERROR] & E_BARRIER));
+}
+#endif
 
 #ifdef __CUDACC__
 // Sums over the W lanes of a group (W = 8, 16 or 32) of eight values a lane: lane l gets the
@@ -534,6 +549,7 @@ struct qz_sim {
     // and the level deposits run on `stream`, and the fork / join events
     cudaStream_t head_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_head = nullptr;
+    cudaEvent_t ev_outcome = nullptr; // the queued head solve's outcome is in h_flags
     bool no_overlap = false; // set by qz_ensemble_step: members stay on one stream
     bool mg_after_direct = false; // the multigrid launch follows a direct solve
     int mg_ppt_floor = 0;    // fewest finest-level points a thread of the head launch takes
@@ -741,7 +757,7 @@ int deposit_segments(qz_sim *s, long m, int bits, int *cell_seg, long ncells_box
                      unsigned **ks_out, int **perm_out, unsigned morton_B);
 // fresh: the accelerations start from zero instead of adding to the arrays; kick_dt != 0:
 // the kick of half a step follows in the same launch
-int gather_head(qz_sim *s, bool fresh = false, double kick_dt = 0.0);
+int gather_head(qz_sim *s, bool fresh = false, double kick_dt = 0.0, const HeadGate &gate = {});
 int kick_drift(qz_sim *s, double dt);
 int kick(qz_sim *s, double dt);
 
@@ -776,7 +792,7 @@ int amr_gather(qz_sim *s, bool fresh = false, double kick_dt = 0.0);
 int poisson_error_head(qz_sim *s, int *converged);
 bool head_one_launch(const qz_sim *s);
 int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued);
-int potential_head_finish(qz_sim *s, cudaStream_t st);
+int potential_head_finish(qz_sim *s);
 int smooth(qz_sim *s, Grid<double> phi, Grid<double> rho, int iters);
 void sync_fine_alt(qz_sim *s);
 void init_kernel_attributes();

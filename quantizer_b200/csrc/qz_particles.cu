@@ -494,11 +494,16 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
                               const double *__restrict__ gx, const double *__restrict__ gy,
                               const double *__restrict__ gz, double *__restrict__ pax,
                               double *__restrict__ pay, double *__restrict__ paz,
-                              int *__restrict__ flags, bool fresh, Kick kick)
+                              int *__restrict__ flags, bool fresh, Kick kick, HeadGate gate)
 {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
+    if (head_failed(gate))
+    {
+        pax[i] = pay[i] = paz[i] = 0.0;
+        return;
+    }
     const double scale = (double)(1 << L);
     double px = x[i] * scale, py = y[i] * scale, pz = z[i] * scale;
     int fx = (int)px, fy = (int)py, fz = (int)pz;
@@ -543,11 +548,11 @@ __global__ void k_gather_head(long n, int L, long D, const double *__restrict__ 
     apply_kick(kick, i, ax, ay, az);
 }
 
-int gather_head(qz_sim *s, bool fresh, double kick_dt)
+int gather_head(qz_sim *s, bool fresh, double kick_dt, const HeadGate &gate)
 {
     if (s->n == 0)
         return QZ_SUCCESS;
-    launch(s, QZ_PROF_GATHER, 72.0 * s->n + 24.0 * s->gpts, k_gather_head, dim3(blocks_for(s->n, 256)), dim3(256), s->n, s->L, s->D, s->x, s->y, s->z, s->gax, s->gay, s->gaz, s->ax, s->ay, s->az, s->flags, fresh, Kick{kick_dt, s->vx, s->vy, s->vz});
+    launch(s, QZ_PROF_GATHER, 72.0 * s->n + 24.0 * s->gpts, k_gather_head, dim3(blocks_for(s->n, 256)), dim3(256), s->n, s->L, s->D, s->x, s->y, s->z, s->gax, s->gay, s->gaz, s->ax, s->ay, s->az, s->flags, fresh, Kick{kick_dt, s->vx, s->vy, s->vz}, gate);
     return check_cuda(cudaGetLastError(), "gather") ? QZ_SUCCESS : QZ_FAILURE;
 }
 

@@ -2482,8 +2482,8 @@ static int head_tail(qz_sim *s, int iter, bool check)
     return QZ_SUCCESS;
 }
 
-// First half of a one-launch head solve: pot_old, the fine-level views and the
-// cooperative launch, all on stream st, with no host wait.  *issued is false
+// First half of a one-launch head solve: pot_old, the fine-level views, the
+// cooperative launch and the read-back of its outcome, all on stream st, with no host wait.  *issued is false
 // (and nothing is queued) when the head solve is not one launch.
 int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued)
 {
@@ -2515,19 +2515,19 @@ int potential_head_issue(qz_sim *s, cudaStream_t st, bool *issued)
                                                 : mg_launch<double>(s, c.max_iter, true, true);
     s->mg_after_direct = false;
     s->stream = keep;
-    *issued = rc == QZ_SUCCESS;
-    return rc;
+    *issued = rc == QZ_SUCCESS &&
+              check_cuda(cudaMemcpyAsync(s->h_flags, s->flags, (F_COUNT + F_OUTST) * sizeof(int),
+                                         cudaMemcpyDeviceToHost, st), "flags") &&
+              check_cuda(cudaEventRecord(s->ev_outcome, st), "multigrid result");
+    return *issued ? QZ_SUCCESS : QZ_FAILURE;
 }
 
-// Second half: waits for the launch on stream st and reads its iteration count,
-// the test's outcome and the barrier status.
-int potential_head_finish(qz_sim *s, cudaStream_t st)
+// Second half: waits for the launch (not for what was queued behind it) and takes its
+// iteration count, the test's outcome and the barrier status.
+int potential_head_finish(qz_sim *s)
 {
     const int *out = s->h_flags + F_COUNT;
-    if (!check_cuda(cudaMemcpyAsync(s->h_flags, s->flags, (F_COUNT + F_OUTST) * sizeof(int),
-                                    cudaMemcpyDeviceToHost, st),
-                    "flags") ||
-        !check_cuda(cudaStreamSynchronize(st), "multigrid result"))
+    if (!check_cuda(cudaEventSynchronize(s->ev_outcome), "multigrid result"))
         return QZ_FAILURE;
     s->mg_ran = out[0];
     s->mg_conv = out[1];
@@ -2550,7 +2550,7 @@ int potential_head(qz_sim *s)
         bool issued = false;
         if (potential_head_issue(s, s->stream, &issued))
             return QZ_FAILURE;
-        return potential_head_finish(s, s->stream);
+        return potential_head_finish(s);
     }
     int iter = 0;
     bool check = false;
