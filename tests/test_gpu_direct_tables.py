@@ -11,7 +11,7 @@ from quantizer_b200 import core, ics
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("lmin", [4, 7])
+@pytest.mark.parametrize("lmin", [4, 6])  # (the cycles behind a 128^3 solve want every SM)
 def test_first_solve_leaves_the_default_stream_alone(lmin):
     ic = ics.plummer(3000, a=0.05, seed=5)
     pots = []
