@@ -780,7 +780,9 @@ __global__ void __launch_bounds__(NT, 1) k_cg_resident(const __grid_constant__ C
                 break;
             // ---- update j + 1
             const double beta = j == 0 ? 0.0 : gamma * inv_g;
-            const double alpha = gamma / (delta - gamma * gamma * inv_ga);
+            // gamma (gamma / ..): gamma alone squared would leave the range of a double where
+            // r.r, whose root is what the caller's units scale, is far from it
+            const double alpha = gamma / (delta - gamma * (gamma * inv_ga));
             until--;
             auto ghost = [&](const u64 (&q)[4], double2 &sg, double2 &at) {
                 sg.x = fma(beta, sg.x, cgr_value(q[0], q[1]));
