@@ -10,6 +10,8 @@
 #include <mutex>
 #include <vector>
 
+#include <cuda.h>
+
 #include "qz_internal.cuh"
 
 namespace qz {
@@ -999,6 +1001,32 @@ __global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L, HeadGa
 // the forces, which a refined step of some 50,000 particles gains from.
 constexpr long HOST_LOADS_MAX = 32768;
 
+// Whether the `bytes` from `mapped`, the device address of page-locked host memory, lie in one
+// allocation or registration: the attributes of a pointer are its first byte's, and a kernel
+// faults where a transfer of an array with a pageable tail ends in an error.
+static bool one_range(const void *mapped, size_t bytes)
+{
+    typedef CUresult (*Query)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        cudaGetLastError();
+        return (Query)f;
+    }();
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[2] = {&start, &size};
+    const CUdeviceptr p = (CUdeviceptr)mapped;
+    return mapped && query && query(2, what, to, p) == CUDA_SUCCESS && start <= p &&
+           p - start <= size && bytes <= size - (p - start);
+}
+
 static int copy_arrays(qz_sim *s, long n, int arrays, const CopyList &L, const HeadGate &gate = {})
 {
     launch(s, QZ_PROF_OTHER, 16.0 * n * arrays, k_copy_arrays, dim3(blocks_for(n, 256), arrays),
@@ -1008,13 +1036,21 @@ static int copy_arrays(qz_sim *s, long n, int arrays, const CopyList &L, const H
 
 extern "C" {
 
+int qz_test_host_range(const void *p, long bytes)
+{
+    cudaPointerAttributes at{};
+    const bool host = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return host && bytes >= 0 && one_range(at.devicePointer, (size_t)bytes) ? 1 : 0;
+}
+
 // One step on host-resident state.  Page-locked arrays (every one of the ten):
 // x..vz and ax..az go in on the simulation's stream, the masses on a second
 // stream beside them and the kick-drift (the deposit is the first stage that
 // reads them), and the drifted positions come back on the second stream
 // while the forces are computed; velocities and accelerations come back after
 // the kick.  Up to HOST_LOADS_MAX particles one kernel moves the arrays in and one
-// moves them out instead.  Pageable arrays: the staged copies of qz_set_particles /
+// moves them out instead, where each array is page-locked as a whole.  Pageable arrays: the staged copies of qz_set_particles /
 // qz_get_particles around qz_step.  The arithmetic is qz_step's either way.
 int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *vx, double *vy,
                  double *vz, const double *m, double *ax, double *ay, double *az)
@@ -1035,7 +1071,8 @@ int qz_step_host(qz_sim *s, double dt, double *x, double *y, double *z, double *
                  at.type == cudaMemoryTypeHost;
         cudaGetLastError();
         mapped[q] = (double *)at.devicePointer;
-        loads = loads && mapped[q] && (uintptr_t)mapped[q] % sizeof(double) == 0;
+        loads = loads && pinned && (uintptr_t)mapped[q] % sizeof(double) == 0 &&
+                one_range(mapped[q], (size_t)n * sizeof(double));
     }
     // outflow boundaries remove particles in the kick-drift: the plain sequence
     if (!pinned || s->cfg.bdry == 2 || n == 0)
