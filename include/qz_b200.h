@@ -481,6 +481,9 @@ QZ_API int qz_test_wait_gives_up(qz_sim *sim, int which, int *out2);
  * rows a block in shared memory and the others in device memory (0: as many as
  * it makes room for); results do not depend on it. */
 QZ_API int qz_test_cg_ghosts(qz_sim *sim, int rows);
+/* qz_test_per_device: how many of a list of devices' calls set up the device (function
+ * attributes are each device's own); needs no device. */
+QZ_API int qz_test_per_device(const int *devices, int n);
 /* qz_test_host_range: 1 when the `bytes` from p are page-locked as a whole, as
  * qz_step_host asks before a kernel reads them. */
 QZ_API int qz_test_host_range(const void *p, long bytes);

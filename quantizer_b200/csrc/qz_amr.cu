@@ -2680,19 +2680,21 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     constexpr int kCgSmem = 40 * 1024; // slot records and cached grid indices
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    static int occ[3] = {0, 0, 0};
-    static std::once_flag occ_once;
-    std::call_once(occ_once, [] {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], (const void *)k_cg_nodes,
-                                                      CG_MAX_THREADS, kCgSmem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], (const void *)k_cg1_nodes,
-                                                      CG_MAX_THREADS, kCgSmem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], (const void *)k_cg2_nodes,
-                                                      CG_MAX_THREADS, kCgSmem);
+    struct Occ {
+        int of[3];
+    };
+    static PerDevice<Occ> occ;
+    const Occ &resident = occ.get(s->device, [] {
+        Occ o{};
+        const void *f[3] = {(const void *)k_cg_nodes, (const void *)k_cg1_nodes,
+                            (const void *)k_cg2_nodes};
+        for (int k = 0; k < 3; k++)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.of[k], f[k], CG_MAX_THREADS, kCgSmem);
+        return o;
     });
     // the overrides and replayed schedules are the two-phase kernel's
     const int variant = (!ov && s->sched_mode != 2) ? c.cg_variant : 0;
-    const int per_sm = occ[variant];
+    const int per_sm = resident.of[variant];
     const bool one = variant >= 1, pipe = variant == 2;
     if (per_sm < 1)
     {
@@ -2730,7 +2732,7 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
         const AmrNode &N = L.h[q];
         const bool cg = !(ov && ov->skip[q]) && (!allow_sor || N.ncells > c.branch_cg_cells);
         onchip[q] = cg && !one && L.cg_ordered && N.nintr > 0 &&
-                    N.nrows <= (long)CG_FILL * CGR_CHUNK_MAX && max_blocks >= CG_FILL;
+                    N.nrows <= (long)CG_FILL * CGR_CHUNK_MAX && cgr_resident(s);
         const long size = (long)(N.rd[0] + 1) * (N.rd[1] + 1) * (N.rd[2] + 1);
         node_cap[q] = replay ? caps[q] : (int)std::min<long>(size, c.max_iter);
     }

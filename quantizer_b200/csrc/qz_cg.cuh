@@ -17,6 +17,9 @@ struct CgrRound {
     double points = 0.0; // interior points of its nodes
 };
 
+// Whether CG_FILL blocks of the solve are resident together on the simulation's device.
+bool cgr_resident(const qz_sim *s);
+
 // Cuts the nodes q with take[q] into chunks and rounds; node_chunk[2q], [2q + 1]
 // become the node's chunk range inside its round.  cap[q]: iteration cap.
 void cgr_plan(const AmrLevel &L, const std::vector<char> &take, const std::vector<int> &cap,

@@ -44,7 +44,6 @@
 // a thread with six index loads (2.5 ms, and 15.3), and every variant with a few spilled
 // registers (the blocks' shared memory leaves little L1 for them).
 #include <algorithm>
-#include <mutex>
 #include <stdio.h>
 #include <string.h>
 
@@ -963,6 +962,25 @@ static const CgrKernel &cgr_kernel(long rows)
     return cgr_kernels[k];
 }
 
+bool cgr_resident(const qz_sim *s)
+{
+    static PerDevice<bool> of;
+    return of.get(s->device, [&] {
+        int sms = 0, k = 0;
+        bool all = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) ==
+                   cudaSuccess;
+        for (const CgrKernel &K : cgr_kernels)
+            all = all &&
+                  cudaFuncSetAttribute(K.f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       CGR_SMEM) == cudaSuccess &&
+                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, K.f, K.threads, CGR_SMEM) ==
+                      cudaSuccess &&
+                  (long)k * sms >= CG_FILL;
+        cudaGetLastError();
+        return all;
+    });
+}
+
 // Rounds run one after another, the nodes of a round side by side.  Nodes of
 // more than one smallest chunk share a round while they fit on chip together (a
 // round's length is mostly the trips through L2, whatever its chunks hold).
@@ -1055,11 +1073,6 @@ int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, cons
 {
     if (rounds.empty())
         return QZ_SUCCESS;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        for (const CgrKernel &k : cgr_kernels)
-            cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, CGR_SMEM);
-    });
     const qz_config &c = s->cfg;
     CgrArgs A;
     memset(&A, 0, sizeof A);

@@ -22,7 +22,6 @@
 // pairs of adjacent x, so that its loads are 128-byte segments; along x, pairs of rows.
 #include <math.h>
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "qz_internal.cuh"
@@ -399,17 +398,25 @@ bool direct_tables(qz_sim *s)
 }
 
 template <int LG>
-static void direct_passes(qz_sim *s, Grid<double> phi, Grid<double> rho, const int *done)
+static bool direct_passes(qz_sim *s, Grid<double> phi, Grid<double> rho, const int *done)
 {
     using S = DirectShape<LG>;
     constexpr int N = S::N;
-    static std::once_flag once;
-    std::call_once(once, [] {
+    static PerDevice<bool> ready;
+    const bool fits = ready.get(s->device, [] {
         const void *f[] = {(const void *)k_sine_x<LG, true>, (const void *)k_sine_x<LG, false>,
                            (const void *)k_sine_yz<LG, true>, (const void *)k_sine_yz<LG, false>};
+        bool ok = true;
         for (const void *k : f)
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)S::SMEM) == cudaSuccess;
+        return ok;
     });
+    if (!fits)
+    {
+        set_error("direct solve: the kernels' shared memory cannot be had");
+        return false;
+    }
     double *w = s->fine_alt_buf;
     const double2 *tw = reinterpret_cast<const double2 *>(s->direct_tab);
     const double *lam = s->direct_tab + 4 * N;
@@ -420,6 +427,7 @@ static void direct_passes(qz_sim *s, Grid<double> phi, Grid<double> rho, const i
     launch_shm(s, QZ_PROF_SMOOTH, 16.0 * pts, S::SMEM, k_sine_yz<LG, true>, g, b, w, tw, lam, done);
     launch_shm(s, QZ_PROF_SMOOTH, 16.0 * pts, S::SMEM, k_sine_yz<LG, false>, g, b, w, tw, lam, done);
     launch_shm(s, QZ_PROF_SMOOTH, 24.0 * pts, S::SMEM, k_sine_x<LG, false>, g, b, phi, rho, w, tw, done);
+    return true;
 }
 
 // Corrects phi (a head grid) to the solution with right-hand side rho and phi's boundary
@@ -428,18 +436,19 @@ static void direct_passes(qz_sim *s, Grid<double> phi, Grid<double> rho, const i
 static int direct_correct_unless(qz_sim *s, double *phi, double *rho, const int *done)
 {
     const Grid<double> p = head_view(s, phi), r = head_view(s, rho);
+    bool ok;
     switch (s->L)
     {
-    case 2: direct_passes<2>(s, p, r, done); break;
-    case 3: direct_passes<3>(s, p, r, done); break;
-    case 4: direct_passes<4>(s, p, r, done); break;
-    case 5: direct_passes<5>(s, p, r, done); break;
-    case 6: direct_passes<6>(s, p, r, done); break;
-    case 7: direct_passes<7>(s, p, r, done); break;
-    case 8: direct_passes<8>(s, p, r, done); break;
-    default: direct_passes<9>(s, p, r, done); break;
+    case 2: ok = direct_passes<2>(s, p, r, done); break;
+    case 3: ok = direct_passes<3>(s, p, r, done); break;
+    case 4: ok = direct_passes<4>(s, p, r, done); break;
+    case 5: ok = direct_passes<5>(s, p, r, done); break;
+    case 6: ok = direct_passes<6>(s, p, r, done); break;
+    case 7: ok = direct_passes<7>(s, p, r, done); break;
+    case 8: ok = direct_passes<8>(s, p, r, done); break;
+    default: ok = direct_passes<9>(s, p, r, done); break;
     }
-    return check_cuda(cudaGetLastError(), "direct solve") ? QZ_SUCCESS : QZ_FAILURE;
+    return ok && check_cuda(cudaGetLastError(), "direct solve") ? QZ_SUCCESS : QZ_FAILURE;
 }
 
 int direct_correct(qz_sim *s, double *phi, double *rho)

@@ -13,6 +13,8 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <map>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -422,6 +424,24 @@ struct AmrNode {
 
 struct AmrChunk {
     int node, begin, end; // [begin, end) of the level's interior list, one node
+};
+
+// A value of each device, made by the first call on it: function attributes, and the
+// occupancies that follow from them, are a device's own, and a process may hold simulations on
+// several (the calls on one run with it as the current device).
+template <typename T> class PerDevice {
+    std::mutex mu;
+    std::map<int, T> of; // its elements stay where they are
+
+public:
+    template <typename Make> const T &get(int device, Make make)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto at = of.find(device);
+        if (at == of.end())
+            at = of.emplace(device, make()).first;
+        return at->second;
+    }
 };
 
 // Stream-ordered allocation context of a simulation: the device's memory pool

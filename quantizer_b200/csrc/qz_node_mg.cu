@@ -832,12 +832,12 @@ static NodeMgBufs &bufs_of(qz_sim *s, int level)
     return s->node_mg->lv[level];
 }
 
-// Cluster size and dynamic shared memory of the launch (set once).
-static int cluster_size(size_t smem)
+// Cluster size of the launch, with its dynamic shared memory (set once per device).
+static int cluster_size(int device)
 {
-    static int cs = 0;
-    static std::once_flag once;
-    std::call_once(once, [&] {
+    static PerDevice<int> of;
+    return of.get(device, [] {
+        int cs = 0;
         cudaFuncSetAttribute((const void *)k_node_mg, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)NMG_SMEM_MAX);
         cudaFuncSetAttribute((const void *)k_node_mg, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -863,9 +863,8 @@ static int cluster_size(size_t smem)
             }
         }
         cudaGetLastError();
+        return cs;
     });
-    (void)smem;
-    return cs;
 }
 
 int node_mg_level(qz_sim *s, AmrLevel &L, int level_index)
@@ -976,7 +975,7 @@ int node_mg_level(qz_sim *s, AmrLevel &L, int level_index)
         set_error("node multigrid buffers");
         return QZ_FAILURE;
     }
-    const int cs = cluster_size(smem);
+    const int cs = cluster_size(s->device);
     if (cs < 1)
     {
         set_error("node multigrid: no cluster of the kernel can be resident");

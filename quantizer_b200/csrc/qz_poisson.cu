@@ -574,15 +574,14 @@ static int smooth_t(qz_sim *s, Grid<T> phi, Grid<T> rho, int iters, Grid<T> scra
         A.iters = iters;
         A.bar = GridBar{s->gbar, s->flags};
         cudaMemsetAsync(s->gbar, 0, 4 * sizeof(unsigned), s->stream);
-        static int per_sm[2] = {0, 0};
-        static std::once_flag once;
-        std::call_once(once, [] {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_cg_smooth<double>, 256, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_cg_smooth<float>, 256, 0);
+        static PerDevice<int> per_sm; // of this T
+        const int ps = per_sm.get(s->device, [] {
+            int k = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_cg_smooth<T>, 256, 0);
+            return k;
         });
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-        const int ps = per_sm[sizeof(T) == 4 ? 1 : 0];
         const long want = ((long)m * m * m + 255) / 256;
         const int blocks = (int)std::max(1L, std::min(want, (long)std::min(ps, 2) * sms));
         if (ps < 1 || blocks > QZ_CG_PART_MAX)
@@ -1826,24 +1825,20 @@ bool mg_persistent(const qz_sim *s)
 }
 
 // Whether one cluster of lc's shape (blocks, threads, shared memory) can be
-// resident on the device: cudaOccupancyMaxActiveClusters once per shape (the
-// first query also allows cluster sizes above the portable 8).
-template <typename T> static bool mg_cluster_fits(const cudaLaunchConfig_t &lc)
+// resident on the device: cudaOccupancyMaxActiveClusters once per device and shape (the
+// query also allows cluster sizes above the portable 8).
+template <typename T> static bool mg_cluster_fits(int device, const cudaLaunchConfig_t &lc)
 {
     static std::mutex mu;
-    static std::vector<std::pair<long, bool>> known; // (blocks << 32 | smem, fits)
-    static bool attr_set = false;
-    const long key = ((long)lc.gridDim.x << 32) | (long)lc.dynamicSmemBytes;
+    static std::vector<std::pair<std::pair<int, long>, bool>> known; // device, blocks << 32 | smem
+    const std::pair<int, long> key(device,
+                                   ((long)lc.gridDim.x << 32) | (long)lc.dynamicSmemBytes);
     std::lock_guard<std::mutex> lock(mu);
     for (const auto &k : known)
         if (k.first == key)
             return k.second;
-    if (!attr_set)
-    {
-        cudaFuncSetAttribute((const void *)k_mg_cycles<T>,
-                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        attr_set = true;
-    }
+    cudaFuncSetAttribute((const void *)k_mg_cycles<T>,
+                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     int nc = 0;
     const bool fits = cudaOccupancyMaxActiveClusters(&nc, (const void *)k_mg_cycles<T>, &lc) ==
                           cudaSuccess &&
@@ -1922,19 +1917,14 @@ static int mg_launch(qz_sim *s, int iters, bool check = false, bool defer = fals
     A.smem = smem <= MG_SMEM_MAX ? 1 : 0;
     if (!A.smem)
         smem = 0;
-    static int per_sm[2] = {0, 0};
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaFuncSetAttribute((const void *)k_mg_cycles<double>,
+    static PerDevice<int> per_sm; // of this T
+    const int ps = per_sm.get(s->device, [] {
+        int k = 0;
+        cudaFuncSetAttribute((const void *)k_mg_cycles<T>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM_MAX);
-        cudaFuncSetAttribute((const void *)k_mg_cycles<float>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM_MAX);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_mg_cycles<double>, MG_THREADS,
-                                                      MG_SMEM_MAX);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_mg_cycles<float>, MG_THREADS,
-                                                      MG_SMEM_MAX);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_mg_cycles<T>, MG_THREADS, MG_SMEM_MAX);
+        return k;
     });
-    const int ps = per_sm[std::is_same<T, float>::value ? 1 : 0];
     if (ps < 1)
     {
         set_error("multigrid kernel cannot be resident");
@@ -2019,7 +2009,7 @@ static int mg_launch(qz_sim *s, int iters, bool check = false, bool defer = fals
         la[0].val.clusterDim.z = 1;
         lc.attrs = la;
         lc.numAttrs = 1;
-        A.cluster = mg_cluster_fits<T>(lc) ? 1 : 0;
+        A.cluster = mg_cluster_fits<T>(s->device, lc) ? 1 : 0;
     }
     void *args[] = {&A};
     cudaEvent_t eb = nullptr, ee = nullptr;

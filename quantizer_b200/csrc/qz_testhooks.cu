@@ -128,6 +128,21 @@ int qz_test_wait_gives_up(qz_sim *s, int which, int *out2)
 
 } // extern "C"
 
+extern "C" QZ_API int qz_test_per_device(const int *devices, int n)
+{
+    if (!devices || n < 0)
+        return -1;
+    PerDevice<int> of;
+    int made = 0;
+    for (int q = 0; q < n; q++)
+        if (of.get(devices[q], [&] {
+                made++;
+                return devices[q];
+            }) != devices[q])
+            return -1;
+    return made;
+}
+
 extern "C" QZ_API int qz_test_cg_ghosts(qz_sim *s, int rows)
 {
     if (!s || rows < 0)
