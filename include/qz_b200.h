@@ -100,12 +100,12 @@ typedef struct qz_config {
     double adjoint_tol;
     /* refinement-node conjugate gradient: 0 (default) the vectors on chip, in
      * registers and shared memory, one exchange an iteration (Chronopoulos-Gear
-     * arrangement; a level whose nodes do not fit, and a node with points on its
-     * grid's faces, runs the reference's two reductions per iteration from
-     * device memory), 1 from device memory with one reduction per iteration (Chronopoulos-Gear arrangement:
-     * the same iterates in exact arithmetic, half the waits), 2 one reduction
-     * per iteration in the pipelined arrangement (Ghysels-Vanroose: w = A r
-     * by recurrence, one stencil and 12 loads a point) */
+     * arrangement; a node that does not fit, or with points on its grid's faces, is
+     * solved as by 3), 1 from device memory with one reduction per iteration
+     * (Chronopoulos-Gear arrangement: the same iterates in exact arithmetic, half
+     * the waits), 2 one reduction per iteration in the pipelined arrangement
+     * (Ghysels-Vanroose: w = A r by recurrence, one stencil and 12 loads a point),
+     * 3 the reference's two reductions per iteration from device memory */
     int cg_variant;
     /* A head solve by red-black Gauss-Seidel V-cycles of at least 100 allowed
      * iterations, with no recorded or replayed schedule, starts with a direct

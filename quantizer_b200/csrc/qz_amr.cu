@@ -2692,8 +2692,9 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o.of[k], f[k], CG_MAX_THREADS, kCgSmem);
         return o;
     });
-    // the overrides and replayed schedules are the two-phase kernel's
-    const int variant = (!ov && s->sched_mode != 2) ? c.cg_variant : 0;
+    // the overrides and replayed schedules are the two-phase kernel's, as is cg_variant 3
+    // (which has no on-chip order)
+    const int variant = (!ov && s->sched_mode != 2) ? c.cg_variant % 3 : 0;
     const int per_sm = resident.of[variant];
     const bool one = variant >= 1, pipe = variant == 2;
     if (per_sm < 1)

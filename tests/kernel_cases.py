@@ -101,8 +101,8 @@ def main() -> None:
                     help="refinement nodes: 0 conjugate gradient, 1 FP32 node multigrid")
     ap.add_argument("--ref-ptcl", type=int, default=9)
     ap.add_argument("--cg-variant", type=int, default=0,
-                    help="node conjugate gradient: 0 two reductions, 1 single reduction, "
-                         "2 pipelined")
+                    help="node conjugate gradient: 0 on chip, 1 single reduction, "
+                         "2 pipelined, 3 two reductions")
     args = ap.parse_args()
     fn = {"smooth": _smooth, "multigrid": _multigrid, "step": _step}[args.what]
     print(json.dumps(fn(args)))
