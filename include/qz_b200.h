@@ -481,6 +481,9 @@ QZ_API int qz_test_wait_gives_up(qz_sim *sim, int which, int *out2);
  * rows a block in shared memory and the others in device memory (0: as many as
  * it makes room for); results do not depend on it. */
 QZ_API int qz_test_cg_ghosts(qz_sim *sim, int rows);
+/* qz_test_cg_scratch: bytes that the on-chip conjugate gradient holds for the
+ * exchange between blocks. */
+QZ_API long qz_test_cg_scratch(const qz_sim *sim);
 /* qz_test_per_device: how many of a list of devices' calls set up the device (function
  * attributes are each device's own); needs no device. */
 QZ_API int qz_test_per_device(const int *devices, int n);

@@ -13,6 +13,7 @@ constexpr int CGR_CHUNK_MIN = 128;   // smallest chunk, in rows
 struct CgrRound {
     int first = 0, count = 0;
     int chunk = 0;       // rows of the largest chunk
+    bool shared = false; // a node of several chunks: blocks that exchange values
     int cap = 0;         // most iterations of a node
     double points = 0.0; // interior points of its nodes
 };

@@ -280,7 +280,7 @@ struct CgrArgs {
     const double *d;
     double *pot, *pot_old;
     u64 *halo[2]; // two words a point of a row
-    u64 *sums[2]; // four words a chunk, CGR_LINE apart
+    u64 *sums[2]; // four words a chunk of a shared round, CGR_LINE apart
     int *status;  // [0] most iterations of a node, [1] a wait gave up, [2] unconverged nodes
     int *iters;
     double tol, tol2, G;
@@ -290,9 +290,9 @@ struct CgrArgs {
     unsigned tag0;
     int chunk; // rows of the largest chunk
     int gcap;  // ghost rows kept in shared memory; the others in spill
-    // scratch of a chunk: per ghost row (6 chunk) its row and the lanes asked for; past
-    // the first GV a thread the ghost half rows' (10 chunk) words, places and s; r of
-    // the ghost rows past gcap
+    // scratch of a chunk of a shared round (the others have no ghosts): per ghost row
+    // (6 chunk) its row and the lanes asked for; past the first GV a thread the ghost half
+    // rows' (10 chunk) words, places and s; r of the ghost rows past gcap
     int2 *grow, *xplace;
     double2 *xs, *spill;
 };
@@ -1051,6 +1051,7 @@ void cgr_plan(const AmrLevel &L, const std::vector<char> &take, const std::vecto
             for (int b = N.row_off; b < N.row_off + N.nrows; b += R.chunk)
                 chunks.push_back({q, b, std::min(b + R.chunk, N.row_off + N.nrows)});
             node_chunk[2 * q + 1] = (int)chunks.size() - R.first;
+            R.shared = R.shared || N.nrows > R.chunk;
             R.cap = std::max(R.cap, cap[q]);
             R.points += N.nintr;
         }
@@ -1099,16 +1100,17 @@ int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, cons
         const int blocks = std::min(R.count, CG_FILL);
         // a node of several chunks has all of them resident at once (cgr_plan)
         const CgrKernel &K = cgr_kernel(R.chunk);
-        const long rows6 = 6L * R.chunk, values = (long)CGR_ROW_GHOSTS * R.chunk;
-        // buffers by the kernel's rows, which a slowly changing tree leaves as they are
-        const long most = (long)K.rows * std::max(R.count, std::min(CG_FILL, R.count * 2));
+        const long rows6 = 6L * R.chunk;
+        // buffers by the kernel's rows, which a slowly changing tree leaves as they are; a
+        // round of one-chunk nodes, whatever their number, exchanges nothing
+        const long most = R.shared ? (long)K.rows * std::min(CG_FILL, R.count * 2) : 0;
         long gcap = std::min(std::min(rows6, R.chunk + 256L), (CGR_SMEM - K.fixed) / CGR_GHOST_BYTES - 1);
         if (s->cgr_ghosts > 0)
             gcap = std::min<long>(gcap, s->cgr_ghosts);
-        if (!cgr_words(s, s->cgr_halo, cgr_room(2 * words)) ||
-            !cgr_words(s, s->cgr_sums, 2L * CGR_LINE * std::max(R.count, CG_FILL)) ||
-            !s->cgr_list.ensure(s->mem, (6 + CGR_ROW_GHOSTS) * most) ||
-            !s->cgr_spill.ensure(s->mem, (2 * CGR_ROW_GHOSTS + 24) * most))
+        if (R.shared && (!cgr_words(s, s->cgr_halo, cgr_room(2 * words)) ||
+                         !cgr_words(s, s->cgr_sums, 2L * CGR_LINE * CG_FILL) ||
+                         !s->cgr_list.ensure(s->mem, (6 + CGR_ROW_GHOSTS) * most) ||
+                         !s->cgr_spill.ensure(s->mem, (2 * CGR_ROW_GHOSTS + 24) * most)))
         {
             set_error("conjugate gradient exchange buffers");
             return QZ_FAILURE;
@@ -1116,24 +1118,29 @@ int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, cons
         const long need = (long)R.cap + 4;
         if (s->cgr_tag < 1 || s->cgr_tag + need >= (1L << 31))
         {
-            cudaMemsetAsync(s->cgr_halo.p, 0, s->cgr_halo.cap * sizeof(u64), s->stream);
-            cudaMemsetAsync(s->cgr_sums.p, 0, s->cgr_sums.cap * sizeof(u64), s->stream);
+            if (s->cgr_halo.p)
+                cudaMemsetAsync(s->cgr_halo.p, 0, s->cgr_halo.cap * sizeof(u64), s->stream);
+            if (s->cgr_sums.p)
+                cudaMemsetAsync(s->cgr_sums.p, 0, s->cgr_sums.cap * sizeof(u64), s->stream);
             s->cgr_tag = 1;
         }
         A.tag0 = (unsigned)s->cgr_tag;
         s->cgr_tag += need;
         A.chunks = v.chunks + R.first;
         A.nchunks = R.count;
-        A.halo[0] = s->cgr_halo.p;
-        A.halo[1] = s->cgr_halo.p + words;
-        A.sums[0] = s->cgr_sums.p;
-        A.sums[1] = s->cgr_sums.p + (long)CGR_LINE * std::max(R.count, CG_FILL);
         A.chunk = R.chunk;
         A.gcap = (int)gcap;
-        A.grow = reinterpret_cast<int2 *>(s->cgr_list.p);
-        A.xplace = A.grow + rows6 * R.count;
-        A.spill = reinterpret_cast<double2 *>(s->cgr_spill.p);
-        A.xs = A.spill + 2 * (rows6 - gcap) * R.count;
+        if (R.shared)
+        {
+            A.halo[0] = s->cgr_halo.p;
+            A.halo[1] = s->cgr_halo.p + words;
+            A.sums[0] = s->cgr_sums.p;
+            A.sums[1] = s->cgr_sums.p + (long)CGR_LINE * CG_FILL;
+            A.grow = reinterpret_cast<int2 *>(s->cgr_list.p);
+            A.xplace = A.grow + rows6 * R.count;
+            A.spill = reinterpret_cast<double2 *>(s->cgr_spill.p);
+            A.xs = A.spill + 2 * (rows6 - gcap) * R.count;
+        }
         const size_t smem = K.fixed + CGR_GHOST_BYTES * gcap;
         cudaEvent_t eb = nullptr, ee = nullptr;
         if (s->prof)

@@ -143,6 +143,11 @@ extern "C" QZ_API int qz_test_per_device(const int *devices, int n)
     return made;
 }
 
+extern "C" QZ_API long qz_test_cg_scratch(const qz_sim *s)
+{
+    return s ? 8 * (s->cgr_halo.cap + s->cgr_sums.cap + s->cgr_list.cap + s->cgr_spill.cap) : -1;
+}
+
 extern "C" QZ_API int qz_test_cg_ghosts(qz_sim *s, int rows)
 {
     if (!s || rows < 0)
