@@ -481,6 +481,9 @@ QZ_API int qz_test_wait_gives_up(qz_sim *sim, int which, int *out2);
  * rows a block in shared memory and the others in device memory (0: as many as
  * it makes room for); results do not depend on it. */
 QZ_API int qz_test_cg_ghosts(qz_sim *sim, int rows);
+/* qz_test_cg_limits: levels of more 4^3-point bricks, and exchanges of more words, than
+ * these count as out of room for the on-chip conjugate gradient (0: as built). */
+QZ_API int qz_test_cg_limits(qz_sim *sim, long bricks, long words);
 /* qz_test_cg_scratch: bytes that the on-chip conjugate gradient holds for the
  * exchange between blocks. */
 QZ_API long qz_test_cg_scratch(const qz_sim *sim);

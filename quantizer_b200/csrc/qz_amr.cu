@@ -1096,11 +1096,10 @@ int amr_build(qz_sim *s)
         C.grid_total = grid_total;
         C.cell_total = cell_total;
         C.cls_total = cls_total;
-        const bool order = s->cfg.node_solver == QZ_NODE_CG && s->cfg.cg_variant == 0;
+        bool order = s->cfg.node_solver == QZ_NODE_CG && s->cfg.cg_variant == 0;
         unsigned long long *bricks = nullptr;
         cg_brick_layout(C);
-        if (order && cg_brick_masks(s, C, &bricks))
-            return QZ_FAILURE;
+        order = order && cg_brick_masks(s, C, &bricks);
         // blocks' numbers of points of each category | their scan | the points' categories
         const int nblk = (int)(cls_total / SEL_THREADS);
         if (!C.box.ensure(s->mem, box_total) || !C.cnt.ensure(s->mem, box_total) ||
@@ -2737,6 +2736,17 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
         const long size = (long)(N.rd[0] + 1) * (N.rd[1] + 1) * (N.rd[2] + 1);
         node_cap[q] = replay ? caps[q] : (int)std::min<long>(size, c.max_iter);
     }
+    std::vector<AmrChunk> chip_chunks;
+    std::vector<int> chip_range(2L * nn, 0);
+    std::vector<CgrRound> rounds;
+    cgr_plan(L, onchip, node_cap, c.cg_chunk_min, chip_chunks, chip_range, rounds);
+    if (!cgr_reserve(s, L, rounds))
+    {
+        // no room for the exchange: every node in memory
+        onchip.assign(nn, 0);
+        chip_chunks.clear();
+        rounds.clear();
+    }
     // Their chunks: the level's other CG points are cut into about CG_FILL chunks
     // (one block a SM), or 2 CG_FILL when a chunk would exceed the CG_UPT points a
     // thread the update phase holds: the slowest SM sets every phase's length, so
@@ -2791,8 +2801,10 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
         node_chunk[2 * q + 1] = (int)L.hchunks.size();
     }
     L.nchunks = (int)L.hchunks.size();
-    std::vector<CgrRound> rounds;
-    cgr_plan(L, onchip, node_cap, c.cg_chunk_min, L.hchunks, node_chunk, rounds);
+    for (int q = 0; q < 2 * nn; q++)
+        if (onchip[q / 2])
+            node_chunk[q] = chip_range[q];
+    L.hchunks.insert(L.hchunks.end(), chip_chunks.begin(), chip_chunks.end());
     if (!sor_nodes.empty() && sor_level(s, L, level_index, sor_nodes))
         return QZ_FAILURE;
     pd = CgPending();
@@ -2836,9 +2848,6 @@ static int cg_level_issue(qz_sim *s, AmrLevel &L, int level_index, CgPending &pd
     {
         CgrSolve v{};
         v.chunks = L.chunks.p + L.nchunks;
-        // the plan's rounds count from the end of the in-memory chunks
-        for (CgrRound &R : rounds)
-            R.first -= L.nchunks;
         v.node_chunk = L.nint.p;
         v.status = L.nint.p + 4 * nn;
         v.iters = L.nint.p + 4 * nn + 3;

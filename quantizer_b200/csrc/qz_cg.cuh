@@ -27,7 +27,10 @@ void cgr_plan(const AmrLevel &L, const std::vector<char> &take, const std::vecto
               long chunk_min, std::vector<AmrChunk> &chunks, std::vector<int> &node_chunk,
               std::vector<CgrRound> &rounds);
 
-// Queues the rounds (chunks: the plan's on the device).
+// Buffers of the exchange between the rounds' blocks; false where they cannot be had.
+bool cgr_reserve(qz_sim *s, const AmrLevel &L, const std::vector<CgrRound> &rounds);
+
+// Queues the rounds (chunks: the plan's on the device) after cgr_reserve.
 struct CgrSolve {
     const AmrChunk *chunks;
     const int *node_chunk;
@@ -44,8 +47,10 @@ int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, cons
 // (brick_mark); the scan of their row counts (brick_base: first row of every
 // brick, then the counts), from which the caller reads the nodes' row ranges; the
 // rows themselves.  cg_order_list does all of it for a one-node level with a list.
+// A level whose masks (cg_brick_masks is false) or rows find no room is left without an
+// order (cg_ordered), and its nodes are solved with their vectors in memory.
 void cg_brick_layout(AmrLevel &L);
-int cg_brick_masks(qz_sim *s, AmrLevel &L, unsigned long long **mask);
+bool cg_brick_masks(qz_sim *s, AmrLevel &L, unsigned long long **mask);
 int cg_brick_scan(qz_sim *s, AmrLevel &L);
 int cg_order(qz_sim *s, AmrLevel &L);
 int cg_order_list(qz_sim *s, AmrLevel &L);

@@ -152,17 +152,20 @@ void cg_brick_layout(AmrLevel &L)
 // Room for `need` elements and what the tree grows by in a few steps.
 static long cgr_room(long need) { return need + need / 4 + 64; }
 
-int cg_brick_masks(qz_sim *s, AmrLevel &L, u64 **mask)
+constexpr long BRICKS_MAX = 1L << 27; // 1 GB of masks
+
+bool cg_brick_masks(qz_sim *s, AmrLevel &L, u64 **mask)
 {
     const long nb = L.brick_total;
-    if (nb > (1L << 27) || !s->brick_mask.ensure(s->mem, nb) || !s->brick_base.ensure(s->mem, 2 * nb + 1))
+    if (nb > (s->cgr_bricks > 0 ? s->cgr_bricks : BRICKS_MAX) || !s->brick_mask.ensure(s->mem, nb) ||
+        !s->brick_base.ensure(s->mem, 2 * nb + 1))
     {
-        set_error("conjugate gradient order buffers");
-        return QZ_FAILURE;
+        cudaGetLastError();
+        return false;
     }
     cudaMemsetAsync(s->brick_mask.p, 0, nb * sizeof(u64), s->stream);
     *mask = s->brick_mask.p;
-    return QZ_SUCCESS;
+    return true;
 }
 
 int cg_brick_scan(qz_sim *s, AmrLevel &L)
@@ -178,8 +181,8 @@ int cg_order(qz_sim *s, AmrLevel &L)
 {
     if (!L.row.ensure(s->mem, cgr_room(L.row_total)) || !L.pos.ensure(s->mem, cgr_room(L.grid_total)))
     {
-        set_error("conjugate gradient order buffers");
-        return QZ_FAILURE;
+        cudaGetLastError();
+        return QZ_SUCCESS;
     }
     cudaMemsetAsync(L.pos.p, 0xff, L.grid_total * sizeof(int), s->stream);
     const long n = 16 * L.brick_total;
@@ -190,14 +193,13 @@ int cg_order(qz_sim *s, AmrLevel &L)
 }
 
 // A one-node level given by its interior list (the head, a host node); left without an
-// order (its node is solved with its vectors in memory) when the list has points
-// on the grid's faces.
+// order, too, when the list has points on the grid's faces.
 int cg_order_list(qz_sim *s, AmrLevel &L)
 {
     u64 *mask;
     L.cg_ordered = false;
-    if (cg_brick_masks(s, L, &mask))
-        return QZ_FAILURE;
+    if (!cg_brick_masks(s, L, &mask))
+        return QZ_SUCCESS;
     const int nb = (int)L.brick_total;
     int *face = s->brick_base.p + 2L * nb;
     cudaMemsetAsync(face, 0, sizeof(int), s->stream);
@@ -1070,6 +1072,28 @@ static bool cgr_words(qz_sim *s, DBuf<u64> &buf, long need)
            check_cuda(cudaMemsetAsync(buf.p, 0, buf.cap * sizeof(u64), s->stream), "cg words");
 }
 
+static long cgr_halo_words(const AmrLevel &L) { return 8L * std::max(L.row_total, 1); }
+
+bool cgr_reserve(qz_sim *s, const AmrLevel &L, const std::vector<CgrRound> &rounds)
+{
+    // by the kernels' rows, which a slowly changing tree leaves as they are; a round of
+    // one-chunk nodes, whatever their number, exchanges nothing
+    long rows = 0;
+    for (const CgrRound &R : rounds)
+        if (R.shared)
+            rows = std::max(rows, (long)cgr_kernel(R.chunk).rows * std::min(CG_FILL, R.count * 2));
+    if (rows == 0)
+        return true;
+    const long halo = cgr_room(2 * cgr_halo_words(L));
+    if ((s->cgr_room == 0 || halo <= s->cgr_room) && cgr_words(s, s->cgr_halo, halo) &&
+        cgr_words(s, s->cgr_sums, 2L * CGR_LINE * CG_FILL) &&
+        s->cgr_list.ensure(s->mem, (6 + CGR_ROW_GHOSTS) * rows) &&
+        s->cgr_spill.ensure(s->mem, (2 * CGR_ROW_GHOSTS + 24) * rows))
+        return true;
+    cudaGetLastError();
+    return false;
+}
+
 int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, const CgrSolve &v)
 {
     if (rounds.empty())
@@ -1094,27 +1118,16 @@ int cgr_launch(qz_sim *s, AmrLevel &L, const std::vector<CgrRound> &rounds, cons
     A.method = v.method;
     A.thr_node = v.thr_node;
     A.cap_node = v.cap_node;
-    const long words = 8L * std::max(L.row_total, 1);
+    const long words = cgr_halo_words(L);
     for (const CgrRound &R : rounds)
     {
         const int blocks = std::min(R.count, CG_FILL);
         // a node of several chunks has all of them resident at once (cgr_plan)
         const CgrKernel &K = cgr_kernel(R.chunk);
         const long rows6 = 6L * R.chunk;
-        // buffers by the kernel's rows, which a slowly changing tree leaves as they are; a
-        // round of one-chunk nodes, whatever their number, exchanges nothing
-        const long most = R.shared ? (long)K.rows * std::min(CG_FILL, R.count * 2) : 0;
         long gcap = std::min(std::min(rows6, R.chunk + 256L), (CGR_SMEM - K.fixed) / CGR_GHOST_BYTES - 1);
         if (s->cgr_ghosts > 0)
             gcap = std::min<long>(gcap, s->cgr_ghosts);
-        if (R.shared && (!cgr_words(s, s->cgr_halo, cgr_room(2 * words)) ||
-                         !cgr_words(s, s->cgr_sums, 2L * CGR_LINE * CG_FILL) ||
-                         !s->cgr_list.ensure(s->mem, (6 + CGR_ROW_GHOSTS) * most) ||
-                         !s->cgr_spill.ensure(s->mem, (2 * CGR_ROW_GHOSTS + 24) * most)))
-        {
-            set_error("conjugate gradient exchange buffers");
-            return QZ_FAILURE;
-        }
         const long need = (long)R.cap + 4;
         if (s->cgr_tag < 1 || s->cgr_tag + need >= (1L << 31))
         {

@@ -655,13 +655,14 @@ struct qz_sim {
     qz::DBuf<int> zone_box;            // a level's zone record (k_zone_roots)
     qz::DBuf<double> seg_mass;         // per deposit segment: mass
     // on-chip conjugate gradient: exchanged words (halo values, partial sums) and the
-    // next launch's first tag, ghost lists, brick scratch; cgr_ghosts (tests) caps the
-    // ghost rows kept in shared memory
+    // next launch's first tag, ghost lists, brick scratch; for tests: caps on the ghost
+    // rows kept in shared memory, the bricks of a level and the words of the exchange
     qz::DBuf<unsigned long long> cgr_halo, cgr_sums, cgr_list, brick_mask;
     qz::DBuf<double> cgr_spill;
     qz::DBuf<int> brick_base;
     long cgr_tag = 0;
     int cgr_ghosts = 0;
+    long cgr_bricks = 0, cgr_room = 0;
     int *h_small = nullptr;            // pinned read-back buffer
     long h_small_cap = 0;
 

@@ -148,6 +148,15 @@ extern "C" QZ_API long qz_test_cg_scratch(const qz_sim *s)
     return s ? 8 * (s->cgr_halo.cap + s->cgr_sums.cap + s->cgr_list.cap + s->cgr_spill.cap) : -1;
 }
 
+extern "C" QZ_API int qz_test_cg_limits(qz_sim *s, long bricks, long words)
+{
+    if (!s || bricks < 0 || words < 0)
+        return QZ_FAILURE;
+    s->cgr_bricks = bricks;
+    s->cgr_room = words;
+    return QZ_SUCCESS;
+}
+
 extern "C" QZ_API int qz_test_cg_ghosts(qz_sim *s, int rows)
 {
     if (!s || rows < 0)
