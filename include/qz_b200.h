@@ -319,7 +319,9 @@ QZ_API int qz_ensemble_step(qz_sim **sims, int nsims, const double *dt, int nste
  * completion) for every combination of host thread count (thread_opts),
  * multigrid points per thread (ppt_opts) and tile core of the tiled multigrid
  * phases (tile_opts: mg_tile values), restoring every simulation's state
- * (particles, accelerations, head potential, statistics) after each trial;
+ * (particles, accelerations, head potential, statistics) after each trial (where no
+ * trial runs multigrid cycles, the heads being solved directly, only the first ppt and
+ * tile options are tried and taken);
  * sets every simulation's mg_points_per_thread and mg_tile to the best
  * combination's and writes the best thread count, points per thread, tile and
  * step time (best_tile may be NULL).  The simulations are left as they were

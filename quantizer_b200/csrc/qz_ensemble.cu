@@ -121,8 +121,16 @@ extern "C" QZ_API int qz_ensemble_autotune(qz_sim **sims, int nsims, const doubl
     }
     int bt = thread_opts[0], bp = ppt_opts[0], bl = tile_opts[0];
     double bms = 1e300;
-    for (int g = 0; g < ntile_opts && rc == QZ_SUCCESS; g++)
-        for (int a = 0; a < nppt_opts && rc == QZ_SUCCESS; a++)
+    auto cycles = [&]() {
+        long long n = 0;
+        for (int k = 0; k < nsims; k++)
+            n += sims[k]->stats.vcycles_total;
+        return n;
+    };
+    const long long cycles0 = cycles();
+    bool ran = true; // a trial ran multigrid cycles
+    for (int g = 0; g < ntile_opts && rc == QZ_SUCCESS && ran; g++)
+        for (int a = 0; a < nppt_opts && rc == QZ_SUCCESS && ran; a++)
         {
             for (int k = 0; k < nsims; k++)
             {
@@ -136,6 +144,10 @@ extern "C" QZ_API int qz_ensemble_autotune(qz_sim **sims, int nsims, const doubl
                 const double ms =
                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0)
                         .count();
+                if (b == nthread_opts - 1)
+                    // the two settings of the cycles' launches do nothing where the direct
+                    // solve leaves no cycle to run: their first options, not the noise's
+                    ran = cycles() > cycles0;
                 if (rc == QZ_SUCCESS && ms < bms)
                 {
                     bms = ms;
