@@ -272,6 +272,31 @@ __device__ __forceinline__ bool cgr_wait2(const u64 *p, u64 (&w)[4], unsigned ta
     return true;
 }
 
+// Waits for a block's sums at p, whose top bit carries its failed test; false when they
+// never came.
+__device__ __forceinline__ bool cgr_wait_sums(const u64 *p, u64 (&w)[4], unsigned tag)
+{
+    constexpr u64 FB = 1ULL << 63;
+    int polls = 0;
+    for (;;)
+    {
+        cgr_load2(p, w);
+        if (cgr_ready(w[0] & ~FB, w[1] & ~FB, tag) && cgr_ready(w[2] & ~FB, w[3] & ~FB, tag))
+            return true;
+        if (++polls > CGR_POLL_LIMIT)
+            return false;
+    }
+}
+
+// Both waits of the solve on words that nothing publishes (they end at their poll limit).
+__global__ void k_cgr_wait_probe(const u64 *words, int *out)
+{
+    u64 w[4];
+    cgr_load2(words, w);
+    out[0] = cgr_wait2(words, w, 5u) ? 1 : 0;
+    out[1] = cgr_wait_sums(words + CGR_LINE, w, 5u) ? 1 : 0;
+}
+
 struct CgrArgs {
     const AmrChunk *chunks; // of this launch; begin, end are rows
     int nchunks;
@@ -698,20 +723,8 @@ __global__ void __launch_bounds__(NT, 1) k_cg_resident(const __grid_constant__ C
                 {
                     const u64 *in = A.sums[j & 1] + (long)(cb + pw * 32 + lane) * CGR_LINE;
                     u64 q[4];
-                    int polls = 0;
-                    constexpr u64 FB = 1ULL << 63;
-                    for (;;)
-                    {
-                        cgr_load2(in, q);
-                        if (cgr_ready(q[0] & ~FB, q[1] & ~FB, tag) &&
-                            cgr_ready(q[2] & ~FB, q[3] & ~FB, tag))
-                            break;
-                        if (++polls > CGR_POLL_LIMIT)
-                        {
-                            sh_lost = 1;
-                            break;
-                        }
-                    }
+                    if (!cgr_wait_sums(in, q, tag))
+                        sh_lost = 1;
                     a = cgr_value(q[0], q[1]);
                     b = cgr_value(q[2], q[3]);
                     f = (int)(q[0] >> 63);
@@ -916,6 +929,28 @@ __global__ void __launch_bounds__(NT, 1) k_cg_resident(const __grid_constant__ C
     }
     if (bad && tid == 0)
         atomicOr(&A.status[1], 1);
+}
+
+int cgr_wait_probe(qz_sim *s, int out[2])
+{
+    u64 *w = nullptr; // two lines of words, then the results
+    const size_t bytes = (2 * CGR_LINE + 1) * sizeof(u64);
+    if (!pool_alloc(s->mem, &w, 2 * CGR_LINE + 1))
+    {
+        set_error("conjugate gradient wait probe: out of device memory");
+        return QZ_FAILURE;
+    }
+    cudaMemsetAsync(w, 0, bytes, s->stream);
+    launch(s, QZ_PROF_OTHER, 0.0, k_cgr_wait_probe, dim3(1), dim3(1), w, (int *)(w + 2 * CGR_LINE));
+    const bool ok = check_cuda(cudaMemcpyAsync(out, w + 2 * CGR_LINE, 2 * sizeof(int),
+                                               cudaMemcpyDeviceToHost, s->stream), "wait probe") &&
+                    check_cuda(cudaStreamSynchronize(s->stream), "wait probe");
+    pool_free(s->mem, w);
+    if (ok && out[0] && out[1])
+        return QZ_SUCCESS;
+    if (ok)
+        set_error("conjugate gradient: a wait for another block's words gave up");
+    return QZ_FAILURE;
 }
 
 // ---- host ---------------------------------------------------------------------------------

@@ -824,6 +824,7 @@ long radix_tiles(long n);
 int scan_exclusive(qz_sim *s, const int *in, int *out, long n);
 int seg_build(qz_sim *s, const unsigned *keys, long n, unsigned morton_B, int *cell_seg);
 int scan_wait_probe(qz_sim *s);
+int cgr_wait_probe(qz_sim *s, int out[2]);
 bool ensure_sort(qz_sim *s, long need); // qz_amr.cu: radix-sort buffers for need pairs
 void scan_set_epoch(qz_sim *s, unsigned epoch);
 

@@ -6,8 +6,10 @@
 //                        epoch wrap)
 //   qz_test_wait_gives_up  runs one bounded wait that cannot be satisfied --
 //                        the scan's look-back on a tile that is never
-//                        published, or the cooperative kernels' grid barrier
-//                        with an arrival count that no block completes -- so
+//                        published, the cooperative kernels' grid barrier
+//                        with an arrival count that no block completes, or the
+//                        on-chip conjugate gradient's waits for a ghost's words
+//                        and for a block's sums that nothing publishes -- so
 //                        that the give-up path (error bit, kernel returns,
 //                        QZ_FAILURE with the message) is exercised without a
 //                        hang: each wait ends after its poll limit (a few
@@ -78,7 +80,7 @@ int qz_test_scan(qz_sim *s, const int *in, int *out, long n, int in_place, unsig
 
 int qz_test_wait_gives_up(qz_sim *s, int which, int *out2)
 {
-    if (!s || (which != 0 && which != 1))
+    if (!s || which < 0 || which > 2)
     {
         set_error("qz_test_wait_gives_up: bad arguments");
         return QZ_FAILURE;
@@ -92,6 +94,17 @@ int qz_test_wait_gives_up(qz_sim *s, int which, int *out2)
         if (out2)
             out2[0] = out2[1] = 0;
         return check_flags(s);
+    }
+    if (which == 2)
+    {
+        int res[2] = {-1, -1};
+        const int rc = cgr_wait_probe(s, res);
+        if (out2)
+        {
+            out2[0] = res[0];
+            out2[1] = res[1];
+        }
+        return rc;
     }
     // barrier words: count, unused, generation, gave-up; then the probe's two results
     unsigned *w = nullptr;
