@@ -489,6 +489,8 @@ QZ_API int qz_test_cg_limits(qz_sim *sim, long bricks, long words);
 /* qz_test_cg_scratch: bytes that the on-chip conjugate gradient holds for the
  * exchange between blocks. */
 QZ_API long qz_test_cg_scratch(const qz_sim *sim);
+/* qz_test_inv_dist: the pair energy's 1 / sqrt(d) of n numbers. */
+QZ_API int qz_test_inv_dist(qz_sim *sim, const double *d, double *out, long n);
 /* qz_test_per_device: how many of a list of devices' calls set up the device (function
  * attributes are each device's own); needs no device. */
 QZ_API int qz_test_per_device(const int *devices, int n);

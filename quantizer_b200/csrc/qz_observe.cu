@@ -263,6 +263,13 @@ __device__ __forceinline__ double inv_dist(double d)
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+__global__ void k_inv_dist(long n, const double *__restrict__ d, double *__restrict__ out)
+{
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        out[i] = inv_dist(d[i]);
+}
+
 // observables.c:77-112: sum over pairs j < i of m_i m_j / |x_i - x_j|.  The triangle is cut
 // into PE_TILE x PE_TILE tiles dealt to a fixed number of blocks (a row of tiles a block
 // would make the last block's row the length of the launch); a thread holds two i and
@@ -454,4 +461,27 @@ extern "C" QZ_API int qz_observables(qz_sim *s, int potential_type, const double
         return QZ_FAILURE;
     }
     return observables(s, potential_type, units, out);
+}
+
+extern "C" QZ_API int qz_test_inv_dist(qz_sim *s, const double *d, double *out, long n)
+{
+    using namespace qz;
+    double *w = nullptr;
+    if (!s || !d || !out || n < 1 || !pool_alloc(s->mem, &w, 2 * n))
+    {
+        set_error("qz_test_inv_dist: bad arguments or out of device memory");
+        return QZ_FAILURE;
+    }
+    bool ok = check_cuda(cudaMemcpyAsync(w, d, n * sizeof(double), cudaMemcpyHostToDevice,
+                                         s->stream), "inv_dist input");
+    if (ok)
+    {
+        launch(s, QZ_PROF_OTHER, 16.0 * n, k_inv_dist, dim3(blocks_for(n, 256)), dim3(256), n, w,
+               w + n);
+        ok = check_cuda(cudaMemcpyAsync(out, w + n, n * sizeof(double), cudaMemcpyDeviceToHost,
+                                        s->stream), "inv_dist output") &&
+             check_cuda(cudaStreamSynchronize(s->stream), "inv_dist");
+    }
+    pool_free(s->mem, w);
+    return ok ? QZ_SUCCESS : QZ_FAILURE;
 }
