@@ -486,6 +486,8 @@ QZ_API int qz_test_cg_ghosts(qz_sim *sim, int rows);
 /* qz_test_cg_limits: levels of more 4^3-point bricks, and exchanges of more words, than
  * these count as out of room for the on-chip conjugate gradient (0: as built). */
 QZ_API int qz_test_cg_limits(qz_sim *sim, long bricks, long words);
+/* qz_test_cg_tag: the next launch's exchange starts at this 31-bit tag. */
+QZ_API int qz_test_cg_tag(qz_sim *sim, long tag);
 /* qz_test_cg_scratch: bytes that the on-chip conjugate gradient holds for the
  * exchange between blocks. */
 QZ_API long qz_test_cg_scratch(const qz_sim *sim);

@@ -145,6 +145,7 @@ def load() -> C.CDLL:
                                        [_P] * 3, C.c_int),
         "qz_test_wait_gives_up": ([vp, C.c_int, _I], C.c_int),
         "qz_test_cg_ghosts": ([vp, C.c_int], C.c_int),
+        "qz_test_cg_tag": ([vp, C.c_long], C.c_int),
         "qz_test_inv_dist": ([vp, _P, _P, C.c_long], C.c_int),
         "qz_test_cg_limits": ([vp, C.c_long, C.c_long], C.c_int),
         "qz_test_cg_scratch": ([vp], C.c_long),

@@ -170,6 +170,16 @@ extern "C" QZ_API int qz_test_cg_limits(qz_sim *s, long bricks, long words)
     return QZ_SUCCESS;
 }
 
+extern "C" QZ_API int qz_test_cg_tag(qz_sim *s, long tag)
+{
+    if (!s || tag < 1 || tag >= 1L << 31)
+        return QZ_FAILURE;
+    if (tag < s->cgr_tag)
+        return QZ_FAILURE; // tags only grow between clearings of the words
+    s->cgr_tag = tag;
+    return QZ_SUCCESS;
+}
+
 extern "C" QZ_API int qz_test_cg_ghosts(qz_sim *s, int rows)
 {
     if (!s || rows < 0)

@@ -1,7 +1,7 @@
 """GPU: the on-chip conjugate gradient on levels of several nodes, against the two-reduction
 kernel in device memory (cg_variant 3): more one-chunk nodes than blocks (a block takes
-several), nodes of different sizes in one round with one-chunk nodes beside them, and nodes
-too large to share a round.
+several), nodes of different sizes in one round with one-chunk nodes beside them, nodes too
+large to share a round, and launches across the wrap of the exchange's 31-bit tags.
 
 Bar of a node: both kernels stop at |r| <= tol rm sqrt(n) (2-norms of the n interior points),
 so their potentials differ by 2 tol rm sqrt(n) / lambda, lambda = (12 / H^2) sin^2(pi H / 2w)
@@ -47,7 +47,7 @@ def _cells(name):
     return 7, np.concatenate([big, far[d > 26]])
 
 
-def _solve(name, variant):
+def _solve(name, variant, tag=None):
     lmin, cells = _cells(name)
     n = len(cells)
     rng = np.random.default_rng(4)
@@ -57,6 +57,10 @@ def _solve(name, variant):
     ic["m"] = rng.uniform(0.5, 1.5, n) / n
     with core.Simulation(ic, lmin, lmax=lmin + 1, ref_ptcl=1, tol=TOL, cg_variant=variant) as sim:
         sim.init_forces()
+        if tag is not None:
+            if tag:
+                core._check(sim.lib.qz_test_cg_tag(sim.h, tag))
+            sim.init_forces()
         nodes = [(sim.node_info(1, q), sim.node_list(1, q, "intr"), sim.node_field(1, q, "pot"))
                  for q in range(sim.num_nodes(1))]
         return nodes, sim.stats().cg_iterations, sim.lib.qz_test_cg_scratch(sim.h), sim.cfg.G, lmin + 1
@@ -78,3 +82,11 @@ def test_levels_of_several_nodes(name, least):
         bar = 2.0 * TOL * rm * root / lam + (ig + iw) * 2.0 ** -53 * 12.0 / H ** 2 * top * root / lam
         assert np.abs(a[pts] - b[pts]).max() <= bar
 
+
+def test_tags_wrap():
+    """The tags start again, on cleared words, when the 31 bits run out: nothing changes."""
+    want = _solve("mixed", 0, tag=0)
+    got = _solve("mixed", 0, tag=2 ** 31 - 2)
+    assert got[1] == want[1]
+    for (_, _, a), (_, _, b) in zip(got[0], want[0]):
+        np.testing.assert_array_equal(a, b)
