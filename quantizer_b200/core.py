@@ -447,7 +447,7 @@ def ensemble_autotune(sims: list, dt, thread_opts=(4, 8, 16, 32, 64), ppt_opts=(
     """Picks the host thread count, multigrid points per thread and tile core of
     the tiled multigrid phases (mg_tile) of the batching form by timing one
     ensemble step per combination (qz_ensemble_autotune; the members' states are
-    put back).  Returns (threads, points_per_thread, mg_tile, ms)."""
+    put back; the cycles' settings only where cycles run).  Returns (threads, points_per_thread, mg_tile, ms)."""
     arr = (C.c_void_p * len(sims))(*[s.h for s in sims])
     d = None if dt is None else np.ascontiguousarray(
         np.broadcast_to(np.asarray(dt, dtype=np.float64), (len(sims),)))

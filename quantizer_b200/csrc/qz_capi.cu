@@ -997,8 +997,9 @@ __global__ void k_copy_arrays(long n, const __grid_constant__ CopyList L, HeadGa
 // Up to this many particles.  A head-only step from page-locked arrays, 32^3 head, us, with
 // transfers and with loads: 2,000 particles 214 and 164, 10,000 245 and 205, 20,000 271 and
 // 237, 40,000 326 and 300, 65,536 386 and 378, 100,000 468 and 483, a million 2,846 and
-// 3,267.  The line lies below the crossing because transfers of the positions back overlap
-// the forces, which a refined step of some 50,000 particles gains from.
+// 3,267.  One line for both kinds of step: it lies below the head-only crossing because
+// transfers of the positions back overlap the forces, which a refined step of some 50,000
+// particles gains from.
 constexpr long HOST_LOADS_MAX = 32768;
 
 // Whether the `bytes` from `mapped`, the device address of page-locked host memory, lie in one
