@@ -55,6 +55,10 @@ int cg_brick_scan(qz_sim *s, AmrLevel &L);
 int cg_order(qz_sim *s, AmrLevel &L);
 int cg_order_list(qz_sim *s, AmrLevel &L);
 
+// Bits of a brick coordinate that the order holds; a level with a longer node (262,144
+// points a side and more) gets no order.
+constexpr int BRICK_BITS = 16;
+
 #ifdef __CUDACC__
 // Marks grid point (x, y, z) of node N in the level's 4^3-point bricks: brick
 // coordinates x / 4, y / 4, z / 4 with their bits interleaved, axes that ran out
@@ -65,7 +69,7 @@ __device__ __forceinline__ void brick_mark(const AmrNode &N, int x, int y, int z
     const unsigned c[3] = {(unsigned)x >> 2, (unsigned)y >> 2, (unsigned)z >> 2};
     unsigned m = 0;
     int sh = 0;
-    for (int b = 0; b < 16; b++)
+    for (int b = 0; b < BRICK_BITS; b++)
         for (int a = 0; a < 3; a++)
             if (b < N.bbits[a])
                 m |= ((c[a] >> b) & 1u) << sh++;

@@ -44,6 +44,7 @@
 // a thread with six index loads (2.5 ms, and 15.3), and every variant with a few spilled
 // registers (the blocks' shared memory leaves little L1 for them).
 #include <algorithm>
+#include <limits.h>
 #include <stdio.h>
 #include <string.h>
 
@@ -116,7 +117,7 @@ __global__ void k_brick_order(long n, int nn, const AmrNode *__restrict__ nodes,
     }
     const AmrNode N = nodes[lo];
     int c[3] = {0, 0, 0}, rest = b - N.brick_off;
-    for (int i = 0; i < 16; i++)
+    for (int i = 0; i < BRICK_BITS; i++)
         for (int a = 0; a < 3; a++)
             if (i < N.bbits[a])
             {
@@ -132,6 +133,7 @@ __global__ void k_brick_order(long n, int nn, const AmrNode *__restrict__ nodes,
 void cg_brick_layout(AmrLevel &L)
 {
     long total = 0;
+    bool wide = false;
     for (AmrNode &N : L.h)
     {
         int bits = 0;
@@ -140,12 +142,13 @@ void cg_brick_layout(AmrLevel &L)
             N.bbits[a] = 0;
             while ((4L << N.bbits[a]) < N.rd[a] + 1)
                 N.bbits[a]++;
+            wide = wide || N.bbits[a] > BRICK_BITS;
             bits += N.bbits[a];
         }
         N.brick_off = (int)total;
         total += 1L << bits;
     }
-    L.brick_total = total;
+    L.brick_total = wide ? LONG_MAX : total;
     L.cg_ordered = false;
 }
 
